@@ -38,11 +38,16 @@ uint64_t dispatch_ws_bytes(int n_entries, int n_expert);
 int launch_dispatch(const int *eid, int n, int n_expert, int se0, int se1, int *ecount, int *eoffs,
                     int *elist, int *pos, void *ws, int *soffs, int s0, int s1, cudaStream_t st, void *plan = nullptr, int D = 0,
                     int FF = 0, int plan_tile_rows = 0);
+// the same with the entries' experts taken from the router, which runs in the first of the launches (idx, wt: outputs);
+// ws: route_dispatch_ws_bytes(T, k, n_expert) bytes
+uint64_t route_dispatch_ws_bytes(int T, int k, int n_expert);
+int launch_route_dispatch(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1, int *idx,
+                          float *wt, int *ecount, int *eoffs, int *elist, int *pos, void *ws, int *soffs, int s0, int s1,
+                          cudaStream_t st, void *plan, int D, int FF, int plan_tile_rows);
+// early: the launch before it in the stream is one of the dispatch launches here (see k_quant_rows)
 int launch_quant(const void *X, int bf16, uint8_t *Xq, uint8_t *Xs, int T, int K, const int *pos,
-                 int k, int shared_row0, bool scatter, cudaStream_t st);
+                 int k, int shared_row0, bool scatter, cudaStream_t st, bool early = false);
 
-// Router + dispatch (+ tensor-core work plan when plan != NULL, + quantise-and-scatter of X when X != NULL)
-// in one single-block launch; T * k <= 1024.
 // decode front end as one thread-block cluster (router, dispatch, plan and the row quantiser in one launch);
 // returns EINVAL without launching when the sizes are outside what it holds
 int launch_front_decode(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int *idx, float *wt,
@@ -55,10 +60,17 @@ int launch_ep_recv_plan(const void *win, uint64_t off_hdr0, uint64_t off_hdr1, u
                         int world, int cap, int row_bytes, int eid_off, unsigned limit, int *status, int n_expert, int se0, int se1,
                         int *ecount, int *eoffs, int *elist, int *pos, int *soffs, int s0, int s1, void *plan, int D, int FF,
                         int plan_tile_rows, int *counts_out, cudaStream_t st);
-int launch_front_small(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1,
-                       int *idx, float *wt, int *ecount, int *eoffs, int *elist, int *pos, int *soffs, int s0, int s1,
-                       void *plan, int D, int FF, int *status, const void *X, int x_is_bf16, uint8_t *Xq, uint8_t *Xs,
-                       int shared_row0, int plan_tile_rows, cudaStream_t st);
+// Router + dispatch (+ tensor-core work plan when plan != NULL) in one cluster launch; front_mid_takes: up to 512 tokens
+bool front_mid_takes(int T, int k, int n_expert);
+int launch_front_mid(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1,
+                     int *idx, float *wt, int *ecount, int *eoffs, int *elist, int *pos, int *soffs, int s0, int s1,
+                     void *plan, int D, int FF, int plan_tile_rows, cudaStream_t st);
+
+// Router, dispatch (+ work plan), scattered row quantiser: everything in front of the expert computation of a batch of any
+// size.  ws: route_dispatch_ws_bytes(T, k, n_expert) bytes; elist may stay unwritten (nothing behind it in a layer reads it)
+int launch_front(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1, int *idx, float *wt,
+                 int *ecount, int *eoffs, int *elist, int *pos, void *ws, int *soffs, int s0, int s1, void *plan, int D, int FF,
+                 int plan_tile_rows, const void *X, int x_is_bf16, uint8_t *Xq, uint8_t *Xs, int shared_row0, cudaStream_t st);
 
 // moe_gemv.cu
 // Sg/Su/Sd + soffs[2]: one extra group (the shared expert) with its own planes and row range, or NULL

@@ -58,7 +58,7 @@ static LayerWs carve(void *base, int T, int E, int k, int D, int FF) {
     w.soffs = (int *)take(8);
     w.elist = (int *)take(n * 4);
     w.pos = (int *)take(n * 4);
-    w.disp = take(dispatch_ws_bytes((int)n, E));
+    w.disp = take(route_dispatch_ws_bytes(T, k <= 8 ? k : 8, E));
     w.Xq = (uint8_t *)take(R * D);
     w.Xs = (uint8_t *)take(R * (D / Q36_QK));
     w.Hq = (uint8_t *)take(R * FF);
@@ -108,32 +108,23 @@ static int layer_impl(const void *Wg, const void *Wu, const void *Wd, const void
     const int n = T * k, R = T * (k + 1);
     int rc;
     const bool use_tc = pick_path(path, T) == Q36_MOE_PATH_TC;
-    const bool fused_front = n <= 1024;
     static const bool no_fuse = getenv("Q36_NOFUSE") != nullptr;
     // decode: gate/up and down in one persistent launch (its plan is cut in token tiles of 16 rows)
     const bool decode_kernel = use_tc && !no_fuse && R <= fused_rows_limit() && ffn_fused_small_fits(R, se1 - se0, D, FF);
     static const bool no_cluster = getenv("Q36_NOCLUSTER") != nullptr;
     // decode on the tensor-core path with every expert resident: one cluster launch does all of the front end
     const bool cluster_front = use_tc && T <= 16 && n <= 128 && se0 == 0 && se1 == E && D % 1024 == 0 && D * T <= 32 * 1024 && !no_cluster;
-    const bool fused_quant = cluster_front || (fused_front && T <= 2);     // beyond a couple of rows the scatter serialises inside one block: measured slower than a launch
+    const int plan_rows = decode_kernel ? 16 : gateup_tile_rows(), sh0 = n, sh1 = shared ? n + T : n;
     if (cluster_front) {
         if ((rc = launch_front_decode(logits, E, k, route_scale, T, logit_stride, w.idx, w.wt, w.ecount, w.eoffs, w.elist,
-                                      w.pos, w.soffs, n, shared ? n + T : n, w.plan, D, FF, w.status, X, x_is_bf16, w.Xq,
+                                      w.pos, w.soffs, sh0, sh1, w.plan, D, FF, w.status, X, x_is_bf16, w.Xq,
                                       w.Xs, shared ? n : -1, k, st)))
             return rc;
-    } else if (fused_front) {
-        if ((rc = launch_front_small(logits, E, k, route_scale, T, logit_stride, se0, se1, w.idx, w.wt, w.ecount, w.eoffs,
-                                     w.elist, w.pos, w.soffs, n, shared ? n + T : n, use_tc ? w.plan : nullptr, D, FF,
-                                     w.status, fused_quant ? X : nullptr, x_is_bf16, w.Xq, w.Xs, shared ? n : -1,
-                                     decode_kernel ? 16 : gateup_tile_rows(), st)))
-            return rc;
-    } else {
-        if ((rc = launch_router_topk(logits, E, k, w.idx, w.wt, route_scale, 1, T, logit_stride, st))) return rc;
-        if ((rc = launch_dispatch(w.idx, n, E, se0, se1, w.ecount, w.eoffs, w.elist, w.pos, w.disp, w.soffs, n,
-                                  shared ? n + T : n, st, use_tc ? w.plan : nullptr, D, FF, decode_kernel ? 16 : gateup_tile_rows())))   // (+ the work plan)
-            return rc;
+    } else if ((rc = launch_front(logits, E, k, route_scale, T, logit_stride, se0, se1, w.idx, w.wt, w.ecount, w.eoffs, w.elist, w.pos,
+                                  w.disp, w.soffs, sh0, sh1, use_tc ? w.plan : nullptr, D, FF, plan_rows, X, x_is_bf16, w.Xq, w.Xs,
+                                  shared ? n : -1, st))) {
+        return rc;
     }
-    if (!fused_quant && (rc = launch_quant(X, x_is_bf16, w.Xq, w.Xs, T, D, w.pos, k, shared ? n : -1, true, st))) return rc;
     const int ng = se1 - se0;
     const int *goffs = w.eoffs + se0;
     // the two grouped-GEMM launches stage their result rows as bf16 for the combine (see ld_y4)

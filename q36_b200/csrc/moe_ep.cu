@@ -494,7 +494,7 @@ static EpWs ep_carve(void *base, int T, int cap, int world, int E, int k, int D,
     w.idx = (int *)take(n * 4); w.wt = (float *)take(n * 4);
     w.ecount = (int *)take((uint64_t)E * 4); w.eoffs = (int *)take((uint64_t)(E + 1) * 4);
     w.elist = (int *)take(n * 4); w.pos = (int *)take(n * 4); w.ypos = (int *)take(n * 4);
-    w.disp = take(dispatch_ws_bytes((int)n, E));
+    w.disp = take(route_dispatch_ws_bytes(T, k, E));
     w.Xq = (uint8_t *)take((uint64_t)T * D); w.Xs = (uint8_t *)take((uint64_t)T * nbs);
     w.reid = (int *)take(S * 4);
     w.lcount = (int *)take((uint64_t)E * 4); w.loffs = (int *)take((uint64_t)(E + 1) * 4);
@@ -603,15 +603,16 @@ static int ep_phase(EpComm *c, int phase, const LayerArgs &a, cudaStream_t st) {
             if ((rc = launch_front_decode(a.logits, E, k, a.route_scale, T, a.logit_stride, w.idx, w.wt, w.ecount, w.eoffs, w.elist,
                                           w.pos, nullptr, 0, 0, nullptr, D, FF, w.status, a.X, a.x_is_bf16, w.Xq, w.Xs, 0, 0, st, &sa)))
                 return rc;
-        } else if (n <= 1024) {
-            if ((rc = launch_front_small(a.logits, E, k, a.route_scale, T, a.logit_stride, 0, E, w.idx, w.wt, w.ecount, w.eoffs,
-                                         w.elist, w.pos, nullptr, 0, 0, nullptr, D, FF, w.status, nullptr, 0, nullptr, nullptr, -1, 0, st)))
-                return rc;
         } else {
-            if ((rc = launch_router_topk(a.logits, E, k, w.idx, w.wt, a.route_scale, 1, T, a.logit_stride, st))) return rc;
-            if ((rc = launch_dispatch(w.idx, n, E, 0, E, w.ecount, w.eoffs, w.elist, w.pos, w.disp, nullptr, 0, 0, st))) return rc;
+            if (front_mid_takes(T, k, E))
+                rc = launch_front_mid(a.logits, E, k, a.route_scale, T, a.logit_stride, 0, E, w.idx, w.wt, w.ecount, w.eoffs, w.elist, w.pos,
+                                      nullptr, 0, 0, nullptr, D, FF, 0, st);
+            else
+                rc = launch_route_dispatch(a.logits, E, k, a.route_scale, T, a.logit_stride, 0, E, w.idx, w.wt, w.ecount, w.eoffs, w.elist,
+                                           w.pos, w.disp, nullptr, 0, 0, st, nullptr, D, FF, 0);
+            if (rc) return rc;
         }
-        if (!cluster_front && (rc = launch_quant(a.X, a.x_is_bf16, w.Xq, w.Xs, T, D, nullptr, 0, 0, true, st))) return rc;
+        if (!cluster_front && (rc = launch_quant(a.X, a.x_is_bf16, w.Xq, w.Xs, T, D, nullptr, 0, 0, true, st, true))) return rc;
         // (larger calls: a kernel of its own.)  Blocks per destination: one up to 256 rows, then one per 256 (at most 32)
         const int nb_send = max(1, min(32, (min(n, C) + 255) / 256));
         if (!cluster_front) launch_k(k_ep_send, dim3(world * nb_send), dim3(1024), 0, st, (const uint8_t *)w.Xq, (const uint8_t *)w.Xs, (const int *)w.idx,

@@ -12,172 +12,280 @@ namespace q36 {
 // One warp per token row; each lane holds n_expert/32 logits in registers.
 // Same selection rule as k_router_topk (q36_ops.cuh:397-431): arg-max on the
 // raw logits, ties to the lower expert id, k rounds with the winner masked.
+//
+// Bound by instruction issue once a few tokens share an SM (two dependent warp reductions and a scan of the lane's eight
+// values per round).  The k-th largest of the 32 lane maxima is a lower bound of the k-th largest logit, and only a
+// dozen logits reach it: those are compacted to one per lane, in expert order, and the rounds run on one value per lane.
+// (Rounds over all eight values per lane: see launch_front for the figures.)
+typedef unsigned long long RouteSlots[32];      // shared memory of a warp: its candidates, key << 32 | expert id
+
+// order-preserving integer key of a float (-0 -> +0: equal floats, equal keys) and back
+__device__ __forceinline__ uint32_t key_of(float v) {
+    const uint32_t b = __float_as_uint(v + 0.f);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float value_of(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
+
 template <int PER_LANE>
 __device__ __forceinline__ void route_row(const float *__restrict__ l, int k, int *idx, float *wt,
-                                          float scale, int renorm, int lane) {
+                                          float scale, int renorm, int lane, RouteSlots &slots) {
+    constexpr uint32_t ALL = 0xffffffffu;
+    const float NONE = -1e30f;           // logits at or below this are never chosen (and -1e30 stands for "no more experts")
+    const uint32_t none = key_of(NONE);
     float v[PER_LANE];
+    uint32_t key[PER_LANE];
 #pragma unroll
     for (int j = 0; j < PER_LANE; j++) v[j] = l[lane + j * 32];
-    float m = -1e30f;
+    uint32_t top = none;
 #pragma unroll
-    for (int j = 0; j < PER_LANE; j++) m = fmaxf(m, v[j]);
-    m = warp_max(m);
+    for (int j = 0; j < PER_LANE; j++) {
+        key[j] = v[j] > NONE ? key_of(v[j]) : none;      // (a NaN is not chosen either)
+        top = max(top, key[j]);
+    }
+    const uint32_t kfirst = __reduce_max_sync(ALL, top);
+    const float m = value_of(kfirst);
     float s = 0.f;
 #pragma unroll
     for (int j = 0; j < PER_LANE; j++) s += expf(v[j] - m);
     s = warp_sum(s);
-    float w_keep = 0.f, wsum = 0.f;  // lane r keeps the weight of round r
-    for (int r = 0; r < k; r++) {
-        float bm = -1e30f;
-        int bj = 0;
+    // the k-th largest lane maximum (several lanes with the same one count as many)
+    uint32_t thr = kfirst;
+    if (PER_LANE > 1) {
+        uint32_t cur = top;
+        for (int left = k; left > 0;) {
+            thr = __reduce_max_sync(ALL, cur);
+            const bool hit = cur == thr;
+            left -= __popc(__ballot_sync(ALL, hit));
+            if (hit) cur = 0;
+        }
+    } else {
+        thr = 0;                         // one value per lane: everybody is a candidate
+    }
+    int base = 0;
 #pragma unroll
-        for (int j = 0; j < PER_LANE; j++)
-            if (v[j] > bm) { bm = v[j]; bj = j; }
-        // warp arg-max in two reductions: the largest value as an order-preserving integer key, then the lowest
-        // expert id among the lanes that hold it (the shuffle tree this replaces was 10 dependent shuffles)
-        const uint32_t bits = __float_as_uint(bm + 0.f);                         // (-0 -> +0: equal floats, equal keys)
-        const uint32_t key = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);
-        const uint32_t kmax = __reduce_max_sync(0xffffffffu, key);
-        const int wi = (int)__reduce_min_sync(0xffffffffu, key == kmax ? (uint32_t)(lane + bj * 32) : 0xffffffffu);
-        const uint32_t vb = (kmax & 0x80000000u) ? (kmax & 0x7fffffffu) : ~kmax;
-        const float wv = __uint_as_float(vb);
-        const float w = expf(wv - m) / s;
-        if (lane == r) { w_keep = w; idx[r] = wi; }
-        wsum += w;
-        if (lane == (wi & 31)) {
+    for (int j = 0; j < PER_LANE; j++) { // slot order = expert order
+        const bool in = key[j] >= thr;
+        const uint32_t mask = __ballot_sync(ALL, in);
+        const int slot = base + __popc(mask & ((1u << lane) - 1u));
+        if (in && slot < 32) slots[slot] = (unsigned long long)key[j] << 32 | (uint32_t)(lane + 32 * j);
+        base += __popc(mask);
+    }
+    __syncwarp();
+    uint32_t k_keep = 0;                 // lane r keeps the choice of round r
+    int i_keep = 0;
+    if (base <= 32) {
+        const unsigned long long c = lane < base ? slots[lane] : 0ull;
+        uint32_t cur = (uint32_t)(c >> 32);
+        int src = 0;
+        for (int r = 0; r < k; r++) {
+            const uint32_t kmax = __reduce_max_sync(ALL, cur);
+            const int who = __ffs(__ballot_sync(ALL, cur == kmax)) - 1;     // the lowest slot = the lowest expert id
+            if (lane == r) src = who;
+            if (lane == who) cur = 0;
+        }
+        k_keep = __shfl_sync(ALL, (uint32_t)(c >> 32), src);
+        i_keep = (int)__shfl_sync(ALL, (uint32_t)c, src);
+    } else {                             // (more than 32 logits tie at the bound: all values, round by round)
+        for (int r = 0; r < k; r++) {
+            uint32_t bk = 0;
+            int bj = 0;
 #pragma unroll
             for (int j = 0; j < PER_LANE; j++)
-                if (j == (wi >> 5)) v[j] = -1e30f;
+                if (key[j] > bk) { bk = key[j]; bj = j; }
+            const uint32_t kmax = __reduce_max_sync(ALL, bk);
+            const int wi = (int)__reduce_min_sync(ALL, bk == kmax ? (uint32_t)(lane + bj * 32) : ALL);
+            if (lane == r) { k_keep = kmax; i_keep = wi; }
+            if (lane == (wi & 31)) {
+#pragma unroll
+                for (int j = 0; j < PER_LANE; j++)
+                    if (j == (wi >> 5)) key[j] = 0;
+            }
         }
     }
-    if (lane < k) wt[lane] = renorm ? (w_keep / wsum * scale) : (w_keep * scale);
+    __syncwarp();                        // (the slots are read: the warp's next row may overwrite them)
+    // the k weights at once, one lane each; their sum in round order
+    const float w_keep = expf(value_of(k_keep) - m) / s;
+    float wsum = 0.f;
+    for (int r = 0; r < k; r++) wsum += __shfl_sync(ALL, w_keep, r);
+    if (lane < k) {
+        idx[lane] = k_keep > none ? i_keep : 0;
+        wt[lane] = renorm ? (w_keep / wsum * scale) : (w_keep * scale);
+    }
+}
+// the row function of a given expert count (32, 64, 128 or 256)
+__device__ __forceinline__ void route_row_of(int n_expert, const float *__restrict__ l, int k, int *idx, float *wt, float scale,
+                                             int renorm, int lane, RouteSlots &slots) {
+    if (n_expert == 256) route_row<8>(l, k, idx, wt, scale, renorm, lane, slots);
+    else if (n_expert == 128) route_row<4>(l, k, idx, wt, scale, renorm, lane, slots);
+    else if (n_expert == 64) route_row<2>(l, k, idx, wt, scale, renorm, lane, slots);
+    else route_row<1>(l, k, idx, wt, scale, renorm, lane, slots);
 }
 
 __global__ void k_router_topk(const float *__restrict__ logits, int n_expert, int k, int *idx,
                               float *wt, float scale, int renorm, int T, int row_stride) {
     Q36_GDS();
+    __shared__ RouteSlots slots[8];
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= T) return;
     const float *l = logits + (size_t)warp * row_stride;
-    if (n_expert == 256) route_row<8>(l, k, idx + (size_t)warp * k, wt + (size_t)warp * k, scale, renorm, lane);
-    else if (n_expert == 128) route_row<4>(l, k, idx + (size_t)warp * k, wt + (size_t)warp * k, scale, renorm, lane);
-    else if (n_expert == 64) route_row<2>(l, k, idx + (size_t)warp * k, wt + (size_t)warp * k, scale, renorm, lane);
-    else route_row<1>(l, k, idx + (size_t)warp * k, wt + (size_t)warp * k, scale, renorm, lane);
+    route_row_of(n_expert, l, k, idx + (size_t)warp * k, wt + (size_t)warp * k, scale, renorm, lane, slots[threadIdx.x >> 5]);
 }
 
 // -------------------------------------------------------------- dispatch
-// Stable counting sort of entry ids by expert in three launches.  Entries are
-// cut into chunks of DISPATCH_CHUNK; inside a chunk warp w owns entries
-// [32w, 32w+32).
-//   k_dispatch_count : per (chunk, expert) counts and each entry's rank among
-//                      the chunk's earlier entries of the same expert
-//   k_dispatch_scan  : per expert exclusive scan over chunks, then over experts
-//   k_dispatch_place : elist / pos from eoffs + chunk base + rank
+// Stable counting sort of entry ids by expert in two launches.  Entries are cut into chunks of at most DISPATCH_CHUNK;
+// inside a chunk warp w owns entries [32w, 32w+32).
+//   k_dispatch_count      : per (expert, chunk) counts and each entry's rank among the chunk's earlier entries of the
+//                           same expert; with ROUTE the chunk's tokens are routed by the same block first
+//   k_dispatch_scan_place : one cluster: per expert exclusive scan over its chunks (a warp per expert), scan over the
+//                           experts, then elist / pos of every entry; its first CTA writes the tensor-core work plan
 // The order inside a bucket is ascending entry id, one of the orders the
 // engine's atomic k_moe_dispatch (q36_engine.cu:3387-3392) can produce.
-constexpr int DISPATCH_CHUNK = 1024;
+// Bound by latency at every size that matters (12 B per entry).  One block that scanned, and separate router and place
+// launches around it, took 46 us at 4096 tokens and 96 at 32,768; see launch_front for the figures now.
+constexpr int DISPATCH_CHUNK = 512;
 constexpr int DISPATCH_MAX_E = 512;
+constexpr int DISPATCH_CLUSTER = 8;
 
-__global__ void __launch_bounds__(DISPATCH_CHUNK)
-k_dispatch_count(const int *__restrict__ eid, int n, int n_expert, int se0, int se1,
-                 int *__restrict__ chunk_cnt, int *__restrict__ lrank) {
-    Q36_GDS();
+// entries per chunk when the router runs in the same block: one token per warp of the block (4096 tokens are then 128
+// blocks; two tokens per warp left half of the chip idle), as far as the chunk holds them
+static inline int route_chunk(int k) { return min(32, DISPATCH_CHUNK / k) * k; }
+
+template <bool ROUTE>
+__global__ void __launch_bounds__(1024)
+k_dispatch_count(const float *__restrict__ logits, int row_stride, int k, float scale, int T, int *__restrict__ idx,
+                 float *__restrict__ wt, const int *__restrict__ eid, int n, int per_chunk, int n_expert, int se0, int se1,
+                 int *__restrict__ cnt_ec, int n_chunk, unsigned short *__restrict__ lrank) {
+    // synchronise first, then let the next grid start: see k_quant_rows
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     __shared__ unsigned short cnt[DISPATCH_CHUNK / 32][DISPATCH_MAX_E];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int i = tid; i < (DISPATCH_CHUNK / 32) * DISPATCH_MAX_E; i += blockDim.x) (&cnt[0][0])[i] = 0;
+    __shared__ int s_idx[DISPATCH_CHUNK];
+    __shared__ float s_wt[DISPATCH_CHUNK];
+    __shared__ RouteSlots slots[ROUTE ? 32 : 1];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, i0 = blockIdx.x * per_chunk;
+    const int ne = min(per_chunk, n - i0), i = i0 + tid;          // entries of this chunk, one thread each (the upper half idles)
+    for (int x = tid; x < (DISPATCH_CHUNK / 32) * DISPATCH_MAX_E / 2; x += blockDim.x) reinterpret_cast<uint32_t *>(&cnt[0][0])[x] = 0;
+    if (ROUTE) {
+        const int t0 = i0 / k, nt = ne / k;
+        for (int t = warp; t < nt; t += 32)
+            route_row_of(n_expert, logits + (size_t)(t0 + t) * row_stride, k, s_idx + t * k, s_wt + t * k, scale, 1, lane, slots[warp]);
+    }
     __syncthreads();
-    const int i = blockIdx.x * DISPATCH_CHUNK + tid;
     int e = -1;
-    if (i < n) {
-        e = eid[i];
+    if (tid < ne) {
+        e = ROUTE ? s_idx[tid] : eid[i];
+        if (ROUTE) { idx[i] = e; wt[i] = s_wt[tid]; }
         if (e < 0 || e < se0 || e >= se1 || e >= n_expert) e = -1;
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, e);
-    const int r_in_warp = __popc(peers & ((1u << lane) - 1u));
-    if (e >= 0 && r_in_warp == 0) cnt[warp][e] = (unsigned short)__popc(peers);
+    int r_in_warp = 0;
+    if (warp < DISPATCH_CHUNK / 32) {
+        const unsigned peers = __match_any_sync(0xffffffffu, e);
+        r_in_warp = __popc(peers & ((1u << lane) - 1u));
+        if (e >= 0 && r_in_warp == 0) cnt[warp][e] = (unsigned short)__popc(peers);
+    }
     __syncthreads();
     for (int x = tid; x < n_expert; x += blockDim.x) {
         int run = 0;
+#pragma unroll
         for (int w = 0; w < DISPATCH_CHUNK / 32; w++) {
             const int c = cnt[w][x];
             cnt[w][x] = (unsigned short)run;
             run += c;
         }
-        chunk_cnt[(size_t)blockIdx.x * n_expert + x] = run;
+        cnt_ec[(size_t)x * n_chunk + blockIdx.x] = run;
     }
     __syncthreads();
-    if (i < n) lrank[i] = (e >= 0) ? (cnt[warp][e] + r_in_warp) : -1;
+    if (tid < ne) lrank[i] = (e >= 0) ? (unsigned short)(cnt[warp][e] + r_in_warp) : (unsigned short)0xffff;
 }
 
-// One block of 1024 threads.  Per-chunk counts -> exclusive prefix per expert over the chunks, in passes of as many
-// chunks as fit in shared memory next to each other (the count table is read and written once, coalesced: a warp per
-// expert going to global memory for every step of its scan took 19 us at 32 chunks x 256 experts); then warp 0 scans
-// the expert totals, and -- when a plan is wanted -- the same block writes the tensor-core work plan of the grouped
-// launches, which depends on nothing else.
-constexpr int SCAN_SMEM_INTS = 8192;   // 32 KB: 32 chunks x 256 experts per pass
+// exclusive block scan of one value per thread (1024 threads); s_w: 32 values of shared memory.  All threads call.
+template <typename V>
+__device__ __forceinline__ V block_scan_excl(V val, V *s_w, V *total) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    V incl = val;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const V u = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += u; }
+    if (lane == 31) s_w[warp] = incl;
+    __syncthreads();
+    V before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 32; w++) { const V u = s_w[w]; if (w < warp) before += u; all += u; }
+    *total = all;
+    return before + incl - val;
+}
+
 __global__ void __launch_bounds__(1024)
-k_dispatch_scan(int *__restrict__ chunk_cnt, int n_chunk, int n_expert, int *__restrict__ ecount, int *__restrict__ eoffs,
-                int *__restrict__ soffs, int s0, int s1, TcPlan *plan, int se0, int se1, int mt_gu, int mt_dn, int plan_tile_rows) {
-    Q36_GDS();
-    __shared__ int s_eoffs[DISPATCH_MAX_E + 1];
+k_dispatch_scan_place(const int *__restrict__ eid, int n, int per_chunk, int n_expert, int *cnt_ec, int n_chunk,
+                      const unsigned short *__restrict__ lrank, int *__restrict__ ecount, int *__restrict__ eoffs,
+                      int *__restrict__ elist, int *__restrict__ pos, int *__restrict__ soffs, int s0, int s1, TcPlan *plan, int se0,
+                      int se1, int mt_gu, int mt_dn, int plan_tile_rows) {
+    // elist == nullptr: the row quantiser behind this launch places the entries itself (k_quant_rows)
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.barrier_arrive();                 // every CTA has started before anyone writes into its shared memory
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    __shared__ int s_tot[DISPATCH_MAX_E], s_eoffs[DISPATCH_MAX_E + 1], s_w[32];
     __shared__ int scratch[4 * (DISPATCH_MAX_GROUPS + 1)];
-    __shared__ int s_tab[SCAN_SMEM_INTS];
-    const int tid = threadIdx.x;
-    for (int x = tid; x < n_expert; x += blockDim.x) s_eoffs[x] = 0;     // running total per expert across the passes
-    __syncthreads();
-    const int cpp = max(1, SCAN_SMEM_INTS / n_expert);                   // chunks per pass
-    for (int c0 = 0; c0 < n_chunk; c0 += cpp) {
-        const int nc = min(cpp, n_chunk - c0), cells = nc * n_expert;
-        for (int i = tid; i < cells; i += blockDim.x) s_tab[i] = chunk_cnt[(size_t)c0 * n_expert + i];
-        __syncthreads();
-        for (int x = tid; x < n_expert; x += blockDim.x) {                // a thread per expert walks the pass's chunks
-            int run = s_eoffs[x];
-            for (int c = 0; c < nc; c++) {
-                const int v = s_tab[c * n_expert + x];
-                s_tab[c * n_expert + x] = run;
-                run += v;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster.block_rank();
+    cluster.barrier_wait();
+    // a warp per expert: exclusive scan over the chunks, in place
+    const int per = (n_expert + DISPATCH_CLUSTER - 1) / DISPATCH_CLUSTER;
+    for (int x = rank * per + warp; x < min(n_expert, (rank + 1) * per); x += 32) {
+        int *row = cnt_ec + (size_t)x * n_chunk;
+        int run = 0;
+        for (int c0 = 0; c0 < n_chunk; c0 += 128) {               // four loads in flight per lane
+            int v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = c0 + 32 * j + lane < n_chunk ? row[c0 + 32 * j + lane] : 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                int incl = v[j];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += u; }
+                if (c0 + 32 * j + lane < n_chunk) row[c0 + 32 * j + lane] = run + incl - v[j];
+                run += __shfl_sync(0xffffffffu, incl, 31);
             }
-            s_eoffs[x] = run;
         }
-        __syncthreads();
-        for (int i = tid; i < cells; i += blockDim.x) chunk_cnt[(size_t)c0 * n_expert + i] = s_tab[i];
-        __syncthreads();
+        if (lane < DISPATCH_CLUSTER) *cluster.map_shared_rank(&s_tot[x], lane) = run;
     }
-    for (int x = tid; x < n_expert; x += blockDim.x) ecount[x] = s_eoffs[x];
+    cluster.sync();   // the totals of every expert are in every CTA; the scanned rows are visible in the cluster
+    int all;
+    const int tot = tid < n_expert ? s_tot[tid] : 0;
+    const int row0 = block_scan_excl(tot, s_w, &all);
+    if (tid < n_expert) s_eoffs[tid] = row0;
+    if (tid == 0) s_eoffs[n_expert] = all;
     __syncthreads();
-    if (tid < 32) {   // exclusive scan of the expert totals: lane owns a contiguous run
-        const int lane = tid;
-        const int per = (n_expert + 31) / 32;
-        int sum = 0;
-        for (int j = 0; j < per; j++) { const int x = lane * per + j; if (x < n_expert) sum += s_eoffs[x]; }
-        int incl = sum;
-        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
-        int run = incl - sum;
-        for (int j = 0; j < per; j++) {
-            const int x = lane * per + j;
-            if (x < n_expert) { const int c = s_eoffs[x]; s_eoffs[x] = run; run += c; }
+    if (rank == 0) {   // the tables, and the work plan, which depends on nothing else
+        if (tid < n_expert) ecount[tid] = tot;
+        if (tid <= n_expert) eoffs[tid] = s_eoffs[tid];
+        if (tid == 0 && soffs) { soffs[0] = s0; soffs[1] = s1; }
+        if (plan) tc_plan_block(s_eoffs + se0, se1 - se0, s1 > s0, s0, s1, plan, mt_gu, mt_dn, scratch, true, plan_tile_rows);
+        return;        // (its shared memory is written by the others before the barrier only)
+    }
+    if (!elist) return;
+    constexpr int U = 4, STEP = (DISPATCH_CLUSTER - 1) * 1024;
+    for (int i0 = (rank - 1) * 1024 + tid; i0 < n; i0 += U * STEP) {
+        int e[U], r[U], b[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int i = i0 + u * STEP;
+            r[u] = i < n ? (int)lrank[i] : 0xffff;
+            e[u] = i < n ? eid[i] : 0;
         }
-        if (lane == 31) s_eoffs[n_expert] = run;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            b[u] = r[u] != 0xffff ? __ldcg(cnt_ec + (size_t)e[u] * n_chunk + (i0 + u * STEP) / per_chunk) : 0;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int i = i0 + u * STEP;
+            if (i >= n) continue;
+            if (r[u] == 0xffff) { pos[i] = -1; continue; }
+            const int p = s_eoffs[e[u]] + b[u] + r[u];
+            elist[p] = i;
+            pos[i] = p;
+        }
     }
-    __syncthreads();
-    for (int x = tid; x <= n_expert; x += blockDim.x) eoffs[x] = s_eoffs[x];
-    if (tid == 0 && soffs) { soffs[0] = s0; soffs[1] = s1; }
-    if (plan) tc_plan_block(s_eoffs + se0, se1 - se0, s1 > s0, s0, s1, plan, mt_gu, mt_dn, scratch, true, plan_tile_rows);
-}
-
-__global__ void k_dispatch_place(const int *__restrict__ eid, int n, int n_expert,
-                                 const int *__restrict__ chunk_base, const int *__restrict__ lrank,
-                                 const int *__restrict__ eoffs, int *__restrict__ elist,
-                                 int *__restrict__ pos) {
-    Q36_GDS();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int r = lrank[i];
-    if (r < 0) { pos[i] = -1; return; }
-    const int e = eid[i];
-    const int p = eoffs[e] + chunk_base[(size_t)(i / DISPATCH_CHUNK) * n_expert + e] + r;
-    elist[p] = i;
-    pos[i] = p;
 }
 
 // ------------------------------------------------------------- quantiser
@@ -298,26 +406,44 @@ __device__ __forceinline__ void quant_block_put(const QStore &qs, int e2, uint8_
     Xs[(size_t)row * (K / Q36_QK) + blk0 + lane] = (uint8_t)(127 + e2);
 }
 
-// warp = (token, run of 32 blocks); K must be a multiple of 1024
-template <bool BF16>
+// warp = (token, run of 32 blocks); K must be a multiple of 1024.
+// early: the token row is read and quantised BEFORE the grid dependency resolves, only its row positions after.  Only
+// for a launch whose predecessor in the stream lets its successor start after it has itself seen everything before it
+// complete (the dispatch kernels above do): the rows were then written by something that is over.
+// PLACE: the kernel also turns every entry's rank into its row (what k_dispatch_scan_place does for callers without this
+// launch): the seven SMs of that cluster took 60 us for the 262,144 entries of 32,768 tokens.
+struct PlaceArgs { const int *idx, *cnt_ec, *eoffs; const unsigned short *lrank; int n_chunk, per_chunk; };
+template <bool BF16, bool PLACE>
 __global__ void __launch_bounds__(256)
 k_quant_rows(const void *__restrict__ X, uint8_t *__restrict__ Xq, uint8_t *__restrict__ Xs, int T, int K,
-             const int *__restrict__ pos, int k, int shared_row0) {
-    Q36_GDS();
+             int *__restrict__ pos, int k, int shared_row0, int early, const PlaceArgs pl) {
+    if (!early) cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     const int runs = K / (32 * Q36_QK);
     const long gwarp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (gwarp >= (long)T * runs) return;
-    const int t = (int)(gwarp / runs), blk = (int)(gwarp % runs) * 32 + lane;
-    int rows[9];
-#pragma unroll
-    for (int d = 0; d < 8; d++) rows[d] = (d < k) ? pos[(size_t)t * k + d] : -1;   // (issued before the row is read)
-    rows[8] = shared_row0 >= 0 ? shared_row0 + t : -1;
+    const bool mine = gwarp < (long)T * runs;
+    const int t = mine ? (int)(gwarp / runs) : 0, run = mine ? (int)(gwarp % runs) : 0, blk = run * 32 + lane;
     const QBlock q = quant_block_lane<BF16>(X, (size_t)t * K + (size_t)blk * Q36_QK);
     const QStore qs = quant_block_pair(q, lane);
+    if (early) cudaGridDependencySynchronize();
+    if (!mine) return;
+    int p = -1;                                      // lane d: the row of the token's entry d
+    if (lane < k) {
+        const int i = t * k + lane;
+        if (PLACE) {
+            const int r = pl.lrank[i], e = pl.idx[i];
+            if (r != 0xffff) p = pl.eoffs[e] + pl.cnt_ec[(size_t)e * pl.n_chunk + i / pl.per_chunk] + r;
+            if (run == 0) pos[i] = p;
+        } else {
+            p = pos[i];
+        }
+    }
 #pragma unroll
-    for (int d = 0; d < 9; d++)
-        if (rows[d] >= 0) quant_block_put(qs, q.e2, Xq, Xs, rows[d], blk - lane, lane, K);
+    for (int d = 0; d < 9; d++) {
+        const int row = d < 8 ? __shfl_sync(0xffffffffu, p, d) : (shared_row0 >= 0 ? shared_row0 + t : -1);
+        if (row >= 0) quant_block_put(qs, q.e2, Xq, Xs, row, blk - lane, lane, K);
+    }
 }
 
 template <bool BF16, bool SCATTER>
@@ -333,10 +459,7 @@ __global__ void k_quant_e4m3(const void *__restrict__ X, uint8_t *__restrict__ X
     quant_task<SCATTER>(quant_load(X, BF16, t, b, K, lane), Xq, Xs, t, b, K, pos, k, shared_row0, lane);
 }
 
-// ------------------------------------------------- fused front end, small T
-// Decode-sized steps spend more time launching the five small kernels above than running them, so for
-// T * k <= FRONT_MAX_ENTRIES one block does router -> dispatch -> (tensor-core work plan) in a single launch.
-// Same results as the separate kernels: the same route_row, the same stable order.
+// ---------------------------------------------------- one-block dispatch of received slots
 constexpr int FRONT_MAX_ENTRIES = 1024;
 
 // Block-wide stable bucketing of up to FRONT_MAX_ENTRIES entries by expert (thread i owns entry i, e = its expert
@@ -397,46 +520,117 @@ __device__ __forceinline__ void sort_entries_block(SortSmem &sm, int e, int n, i
     if (plan) tc_plan_block(sm.s_eoffs + se0, se1 - se0, s1 > s0, s0, s1, plan, mt_gu, mt_dn, sm.scratch, false, plan_tile_rows);
 }
 
+// ------------------------------------------------- front end of up to 512 tokens: one cluster
+// Router -> stable dispatch -> work plan in ONE launch.  CTA r of the cluster routes the tokens [r tpc, (r + 1) tpc) and
+// counts its entries per expert; the counts (2 B each) go to every CTA's shared memory, so that each of them knows every
+// expert's offset after one cluster barrier and places its own entries.
+// Bound by latency: logits (one read), eight dependent selection rounds, three block barriers and a cluster barrier.
+// One block that did all of it took 21 us at 33 tokens and 23 at 96 (the k_front_small this replaces), five launches
+// 28 us at 300; see launch_front for the figures now.
+constexpr int FM_CLUSTER = 8;
+constexpr int FM_ENTRIES = 512;                       // per CTA
+constexpr int FM_MAX_E = 256;                         // what the router takes
+
 __global__ void __launch_bounds__(1024)
-k_front_small(const float *__restrict__ logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1,
-              int *__restrict__ idx, float *__restrict__ wt, int *__restrict__ ecount, int *__restrict__ eoffs,
-              int *__restrict__ elist, int *__restrict__ pos, int *__restrict__ soffs, int s0, int s1,
-              TcPlan *plan, int mt_gu, int mt_dn, const void *__restrict__ X, int x_is_bf16,
-              uint8_t *__restrict__ Xq, uint8_t *__restrict__ Xs, int D, int shared_row0, int plan_tile_rows) {
-    Q36_GDS();
-    __shared__ SortSmem sm;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarp = blockDim.x >> 5;
-    const int n = T * k;
-    const int used_warps = (n + 31) / 32;
-    for (int i = tid; i < used_warps * DISPATCH_MAX_E; i += blockDim.x) (&sm.cnt[0][0])[i] = 0;
-    for (int t = warp; t < T; t += nwarp) {
-        const float *l = logits + (size_t)t * row_stride;
-        int *ix = idx + (size_t)t * k;
-        float *w = wt + (size_t)t * k;
-        if (n_expert == 256) route_row<8>(l, k, ix, w, scale, 1, lane);
-        else if (n_expert == 128) route_row<4>(l, k, ix, w, scale, 1, lane);
-        else if (n_expert == 64) route_row<2>(l, k, ix, w, scale, 1, lane);
-        else route_row<1>(l, k, ix, w, scale, 1, lane);
+k_front_mid(const float *__restrict__ logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1,
+            int *__restrict__ idx, float *__restrict__ wt, int *__restrict__ ecount, int *__restrict__ eoffs,
+            int *__restrict__ elist, int *__restrict__ pos, int *__restrict__ soffs, int s0, int s1, TcPlan *plan, int mt_gu,
+            int mt_dn, int plan_tile_rows) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.barrier_arrive();                 // every CTA has started before anyone writes into its shared memory
+    // synchronise first, then let the next grid start: see k_quant_rows
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    __shared__ unsigned short cnt[FM_ENTRIES / 32][FM_MAX_E];    // per (entry warp, expert): count, then base
+    __shared__ unsigned short s_cta[FM_CLUSTER][FM_MAX_E];       // entries of every CTA per expert
+    __shared__ int s_idx[FM_ENTRIES], s_base[FM_MAX_E];
+    __shared__ float s_wt[FM_ENTRIES];
+    __shared__ RouteSlots slots[32];
+    __shared__ unsigned long long s_w[32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = (int)cluster.block_rank();
+    const int tpc = (T + FM_CLUSTER - 1) / FM_CLUSTER, t0 = min(T, rank * tpc), nt = min(tpc, T - t0), ne = nt * k;
+    const int used_warps = (ne + 31) / 32;
+    for (int x = tid; x < used_warps * FM_MAX_E / 2; x += 1024) reinterpret_cast<uint32_t *>(&cnt[0][0])[x] = 0;
+    for (int t = warp; t < nt; t += 32)
+        route_row_of(n_expert, logits + (size_t)(t0 + t) * row_stride, k, s_idx + t * k, s_wt + t * k, scale, 1, lane, slots[warp]);
+    __syncthreads();
+    int e = -1;
+    const int i = t0 * k + tid;
+    if (tid < ne) {
+        e = s_idx[tid];
+        idx[i] = e;
+        wt[i] = s_wt[tid];
+        if (e < se0 || e >= se1 || e >= n_expert) e = -1;
     }
-    __syncthreads();   // idx written by this block is visible to it after the barrier
-    sort_entries_block(sm, tid < n ? idx[tid] : -1, n, n_expert, se0, se1, ecount, eoffs, elist, pos, soffs, s0, s1, plan, mt_gu,
-                       mt_dn, plan_tile_rows);
-    if (X) {   // decode: quantise and scatter the T rows here as well (pos[] of this block is visible after the barrier)
-        __syncthreads();
-        const int nbk = D / Q36_QK;
-        const int ntask = T * nbk;
-        for (int base = warp; base < ntask; base += 8 * nwarp) {   // eight loads in flight per lane
-            float v[8];
+    int r_in_warp = 0;
+    if (warp < used_warps) {
+        const unsigned peers = __match_any_sync(0xffffffffu, e);
+        r_in_warp = __popc(peers & ((1u << lane) - 1u));
+        if (e >= 0 && r_in_warp == 0) cnt[warp][e] = (unsigned short)__popc(peers);
+    }
+    __syncthreads();
+    cluster.barrier_wait();
+    if (tid < n_expert) {
+        int run = 0;
+        for (int w = 0; w < used_warps; w++) {
+            const int c = cnt[w][tid];
+            cnt[w][tid] = (unsigned short)run;
+            run += c;
+        }
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const int task = base + j * nwarp;
-                v[j] = (task < ntask) ? quant_load(X, x_is_bf16 != 0, task / nbk, task % nbk, D, lane) : 0.f;
-            }
+        for (int r = 0; r < FM_CLUSTER; r++) *cluster.map_shared_rank(&s_cta[rank][tid], r) = (unsigned short)run;
+    }
+    cluster.sync();
+    // rows, gate/up token tiles and down token tiles before every expert, in one scan
+    const int tr_gu = plan_tile_rows ? plan_tile_rows : TC_N_GATEUP, tr_dn = plan_tile_rows ? plan_tile_rows : TC_N_DOWN;
+    int tot = 0, mine = 0;
+    if (tid < n_expert) {
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const int task = base + j * nwarp;
-                if (task < ntask) quant_task<true>(v[j], Xq, Xs, task / nbk, task % nbk, D, pos, k, shared_row0, lane);
+        for (int r = 0; r < FM_CLUSTER; r++) {
+            const int c = s_cta[r][tid];
+            if (r < rank) mine += c;
+            tot += c;
+        }
+    }
+    typedef unsigned long long u64;
+    u64 all;
+    const u64 excl = block_scan_excl<u64>((u64)tot | (u64)((tot + tr_gu - 1) / tr_gu) << 20 | (u64)((tot + tr_dn - 1) / tr_dn) << 40, s_w, &all);
+    const int row0 = (int)(excl & 0xfffff);
+    if (tid < n_expert) s_base[tid] = row0 + mine;
+    __syncthreads();
+    if (tid < ne) {
+        int p = -1;
+        if (e >= 0) {
+            p = s_base[e] + cnt[warp][e] + r_in_warp;
+            elist[p] = i;
+        }
+        pos[i] = p;
+    }
+    if (rank != 0) return;
+    if (tid < n_expert) {
+        ecount[tid] = tot;
+        eoffs[tid] = row0;
+        if (plan && tid >= se0 && tid < se1) {   // (groups here hold a few token tiles at most: ranking them by size would buy nothing)
+            const int g = tid - se0;
+            plan->row0[g] = row0; plan->cnt[g] = tot; plan->done[g] = 0; plan->order[g] = g;
+            plan->base[0][g] = (int)(excl >> 20 & 0xfffff) * mt_gu; plan->base[1][g] = (int)(excl >> 40) * mt_dn;
+        }
+    }
+    if (tid == 0) {
+        eoffs[n_expert] = (int)(all & 0xfffff);
+        if (soffs) { soffs[0] = s0; soffs[1] = s1; }
+        if (plan) {
+            int G = se1 - se0, ta = (int)(all >> 20 & 0xfffff) * mt_gu, tb = (int)(all >> 40) * mt_dn;
+            if (s1 > s0) {                       // the shared expert's rows are one more group
+                plan->row0[G] = s0; plan->cnt[G] = s1 - s0; plan->done[G] = 0; plan->order[G] = G;
+                plan->base[0][G] = ta; plan->base[1][G] = tb;
+                ta += (s1 - s0 + tr_gu - 1) / tr_gu * mt_gu;
+                tb += (s1 - s0 + tr_dn - 1) / tr_dn * mt_dn;
+                G++;
             }
+            plan->base[0][G] = ta; plan->base[1][G] = tb;
+            plan->n_tiles[0] = ta; plan->n_tiles[1] = tb; plan->n_groups = G; plan->gu_done = 0; plan->tile_rows = plan_tile_rows;
         }
     }
 }
@@ -503,15 +697,15 @@ int launch_ep_recv_plan(const void *win, uint64_t off_hdr0, uint64_t off_hdr1, u
     return check_launch();
 }
 
-int launch_front_small(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1,
-                       int *idx, float *wt, int *ecount, int *eoffs, int *elist, int *pos, int *soffs, int s0, int s1,
-                       void *plan, int D, int FF, int *status, const void *X, int x_is_bf16, uint8_t *Xq, uint8_t *Xs,
-                       int shared_row0, int plan_tile_rows, cudaStream_t st) {
-    if (T * k > FRONT_MAX_ENTRIES || n_expert > DISPATCH_MAX_E) return Q36_MOE_EINVAL;
-    (void)status;   // (sticky status words: nothing to clear here)
-    launch_k(k_front_small, dim3(1), dim3(1024), 0, st, logits, n_expert, k, scale, T, row_stride, se0, se1, idx, wt,
-             ecount, eoffs, elist, pos, soffs, s0, s1, (TcPlan *)plan, FF / TC_M, D / TC_M, X, x_is_bf16, Xq, Xs, D,
-             shared_row0, plan_tile_rows);
+bool front_mid_takes(int T, int k, int n_expert) {
+    return k >= 1 && k <= 8 && n_expert <= FM_MAX_E && (T + FM_CLUSTER - 1) / FM_CLUSTER * k <= FM_ENTRIES;
+}
+int launch_front_mid(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1,
+                     int *idx, float *wt, int *ecount, int *eoffs, int *elist, int *pos, int *soffs, int s0, int s1,
+                     void *plan, int D, int FF, int plan_tile_rows, cudaStream_t st) {
+    if (!front_mid_takes(T, k, n_expert)) return Q36_MOE_EINVAL;
+    launch_k_cluster(k_front_mid, dim3(1, 1, FM_CLUSTER), dim3(1024), FM_CLUSTER, st, logits, n_expert, k, scale, T, row_stride, se0, se1,
+                     idx, wt, ecount, eoffs, elist, pos, soffs, s0, s1, (TcPlan *)plan, FF / TC_M, D / TC_M, plan_tile_rows);
     return check_launch();
 }
 
@@ -586,15 +780,13 @@ k_front_decode(const float *__restrict__ logits, int n_expert, int k, float scal
     __shared__ unsigned short cnt[FD_MAX_ENTRIES / 32][DISPATCH_MAX_E];   // per (entry warp, expert): count, then base
     __shared__ int s_idx[FD_MAX_ENTRIES];
     __shared__ float s_wt[FD_MAX_ENTRIES];
+    __shared__ RouteSlots slots[16];                                      // one warp per token, at most 16
     __shared__ int s_eoffs[DISPATCH_MAX_E + 1];
     __shared__ int s_wsum[FD_THREADS / 32];
     const int used_warps = (n + 31) / 32;
     if (warp < T) {
         const float *l = logits + (size_t)warp * row_stride;
-        if (n_expert == 256) route_row<8>(l, k, s_idx + warp * k, s_wt + warp * k, scale, 1, lane);
-        else if (n_expert == 128) route_row<4>(l, k, s_idx + warp * k, s_wt + warp * k, scale, 1, lane);
-        else if (n_expert == 64) route_row<2>(l, k, s_idx + warp * k, s_wt + warp * k, scale, 1, lane);
-        else route_row<1>(l, k, s_idx + warp * k, s_wt + warp * k, scale, 1, lane);
+        route_row_of(n_expert, l, k, s_idx + warp * k, s_wt + warp * k, scale, 1, lane, slots[warp]);
     } else {
         for (int i = tid - 32 * T; i < used_warps * DISPATCH_MAX_E; i += FD_THREADS - 32 * T) (&cnt[0][0])[i] = 0;
     }
@@ -739,34 +931,88 @@ int launch_router_topk(const float *logits, int n_expert, int k, int *idx, float
     return check_launch();
 }
 
+// [expert][chunk] counts, then the entries' ranks
 uint64_t dispatch_ws_bytes(int n_entries, int n_expert) {
     const uint64_t n_chunk = ((uint64_t)n_entries + DISPATCH_CHUNK - 1) / DISPATCH_CHUNK;
-    return (n_chunk * n_expert + (uint64_t)n_entries) * sizeof(int) + 256;
+    return n_chunk * n_expert * sizeof(int) + (uint64_t)n_entries * sizeof(unsigned short) + 256;
+}
+uint64_t route_dispatch_ws_bytes(int T, int k, int n_expert) {
+    const uint64_t n_chunk = ((uint64_t)T * k + route_chunk(k) - 1) / route_chunk(k);
+    return n_chunk * n_expert * sizeof(int) + (uint64_t)T * k * sizeof(unsigned short) + 256;
 }
 
+// eid == nullptr: the entries are the top-k experts of `logits`, written to idx / wt (per_chunk: whole tokens)
+static int dispatch_launches(const float *logits, int row_stride, int k, float scale, int T, int *idx, float *wt, const int *eid, int n,
+                             int n_expert, int se0, int se1, int *ecount, int *eoffs, int *elist, int *pos, void *ws, int *soffs, int s0,
+                             int s1, cudaStream_t st, void *plan, int D, int FF, int plan_tile_rows) {
+    const int per_chunk = eid ? DISPATCH_CHUNK : route_chunk(k), n_chunk = (n + per_chunk - 1) / per_chunk;
+    int *cnt_ec = (int *)ws;
+    unsigned short *lrank = (unsigned short *)(cnt_ec + (size_t)n_chunk * n_expert);
+    if (n > 0) {
+        if (eid) launch_k(k_dispatch_count<false>, dim3(n_chunk), dim3(1024), 0, st, logits, row_stride, k, scale, T, idx, wt, eid, n, per_chunk,
+                          n_expert, se0, se1, cnt_ec, n_chunk, lrank);
+        else launch_k(k_dispatch_count<true>, dim3(n_chunk), dim3(1024), 0, st, logits, row_stride, k, scale, T, idx, wt, eid, n, per_chunk,
+                      n_expert, se0, se1, cnt_ec, n_chunk, lrank);
+    }
+    launch_k_cluster(k_dispatch_scan_place, dim3(1, 1, DISPATCH_CLUSTER), dim3(1024), DISPATCH_CLUSTER, st, eid ? eid : (const int *)idx, n,
+                     per_chunk, n_expert, cnt_ec, n_chunk, (const unsigned short *)lrank, ecount, eoffs, elist, pos, soffs, s0, s1,
+                     (TcPlan *)plan, se0, se1, plan ? FF / TC_M : 0, plan ? D / TC_M : 0, plan_tile_rows);
+    return check_launch();
+}
 int launch_dispatch(const int *eid, int n, int n_expert, int se0, int se1, int *ecount, int *eoffs,
                     int *elist, int *pos, void *ws, int *soffs, int s0, int s1, cudaStream_t st, void *plan, int D, int FF,
                     int plan_tile_rows) {
-    const int n_chunk = (n + DISPATCH_CHUNK - 1) / DISPATCH_CHUNK;
-    int *chunk_cnt = (int *)ws;
-    int *lrank = chunk_cnt + (size_t)n_chunk * n_expert;
-    if (n > 0) launch_k(k_dispatch_count, dim3(n_chunk), dim3(DISPATCH_CHUNK), 0, st, eid, n, n_expert, se0, se1, chunk_cnt, lrank);
-    launch_k(k_dispatch_scan, dim3(1), dim3(1024), 0, st, chunk_cnt, n_chunk, n_expert, ecount, eoffs, soffs, s0, s1, (TcPlan *)plan,
-             se0, se1, plan ? FF / TC_M : 0, plan ? D / TC_M : 0, plan_tile_rows);
-    if (n > 0) launch_k(k_dispatch_place, dim3((n + 255) / 256), dim3(256), 0, st, eid, n, n_expert, chunk_cnt, lrank, eoffs, elist, pos);
+    return dispatch_launches(nullptr, 0, 1, 0.f, 0, nullptr, nullptr, eid, n, n_expert, se0, se1, ecount, eoffs, elist, pos, ws, soffs, s0,
+                             s1, st, plan, D, FF, plan_tile_rows);
+}
+int launch_route_dispatch(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1, int *idx,
+                          float *wt, int *ecount, int *eoffs, int *elist, int *pos, void *ws, int *soffs, int s0, int s1,
+                          cudaStream_t st, void *plan, int D, int FF, int plan_tile_rows) {
+    return dispatch_launches(logits, row_stride, k, scale, T, idx, wt, nullptr, T * k, n_expert, se0, se1, ecount, eoffs, elist, pos, ws,
+                             soffs, s0, s1, st, plan, D, FF, plan_tile_rows);
+}
+
+static bool quant_rows_takes(int K, int k) { return K % (32 * Q36_QK) == 0 && k <= 8; }
+template <bool PLACE>
+static void launch_quant_rows(const void *X, int bf16, uint8_t *Xq, uint8_t *Xs, int T, int K, int *pos, int k, int shared_row0,
+                              bool early, const PlaceArgs &pl, cudaStream_t st) {
+    const unsigned grid = (unsigned)(((long)T * (K / (32 * Q36_QK)) + 7) / 8);
+    if (bf16) launch_k(k_quant_rows<true, PLACE>, dim3(grid), dim3(256), 0, st, X, Xq, Xs, T, K, pos, k, shared_row0, early ? 1 : 0, pl);
+    else launch_k(k_quant_rows<false, PLACE>, dim3(grid), dim3(256), 0, st, X, Xq, Xs, T, K, pos, k, shared_row0, early ? 1 : 0, pl);
+}
+// Router, dispatch, plan and the scattered row quantiser of a batch of any size.  Up to 512 tokens one cluster (k_front_mid)
+// in front of the quantiser, else the routing count, the scan and the quantiser, which places the entries.
+// Measured (us, router to quantised rows, 256 experts, top-8): 33 tokens 9 against 18 with the kernels this replaces, 96
+// tokens 8 against 22, 300 tokens 15 against 24, 1001 tokens 23 against 31, 4096 tokens 33 against 47.
+int launch_front(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1, int *idx, float *wt,
+                 int *ecount, int *eoffs, int *elist, int *pos, void *ws, int *soffs, int s0, int s1, void *plan, int D, int FF,
+                 int plan_tile_rows, const void *X, int x_is_bf16, uint8_t *Xq, uint8_t *Xs, int shared_row0, cudaStream_t st) {
+    int rc;
+    if (front_mid_takes(T, k, n_expert)) {
+        if ((rc = launch_front_mid(logits, n_expert, k, scale, T, row_stride, se0, se1, idx, wt, ecount, eoffs, elist, pos, soffs, s0, s1,
+                                   plan, D, FF, plan_tile_rows, st)))
+            return rc;
+        return launch_quant(X, x_is_bf16, Xq, Xs, T, D, pos, k, shared_row0, true, st, true);
+    }
+    const bool place = quant_rows_takes(D, k);
+    if ((rc = launch_route_dispatch(logits, n_expert, k, scale, T, row_stride, se0, se1, idx, wt, ecount, eoffs, place ? nullptr : elist,
+                                    pos, ws, soffs, s0, s1, st, plan, D, FF, plan_tile_rows)))
+        return rc;
+    if (!place) return launch_quant(X, x_is_bf16, Xq, Xs, T, D, pos, k, shared_row0, true, st, true);
+    const int per_chunk = route_chunk(k), n_chunk = (T * k + per_chunk - 1) / per_chunk;
+    const int *cnt_ec = (const int *)ws;
+    launch_quant_rows<true>(X, x_is_bf16, Xq, Xs, T, D, pos, k, shared_row0, true,
+                            PlaceArgs{idx, cnt_ec, eoffs, (const unsigned short *)(cnt_ec + (size_t)n_chunk * n_expert), n_chunk, per_chunk}, st);
     return check_launch();
 }
 
 int launch_quant(const void *X, int bf16, uint8_t *Xq, uint8_t *Xs, int T, int K, const int *pos,
-                 int k, int shared_row0, bool scatter, cudaStream_t st) {
+                 int k, int shared_row0, bool scatter, cudaStream_t st, bool early) {
     if (T <= 0) return Q36_MOE_OK;
     const long warps = (long)T * (K / Q36_QK);
     const unsigned grid = (unsigned)((warps + 7) / 8);
-    if (scatter && K % (32 * Q36_QK) == 0 && k <= 8) {
-        const long w2 = (long)T * (K / (32 * Q36_QK));
-        const unsigned g2 = (unsigned)((w2 + 7) / 8);
-        if (bf16) launch_k(k_quant_rows<true>, dim3(g2), dim3(256), 0, st, X, Xq, Xs, T, K, pos, k, shared_row0);
-        else launch_k(k_quant_rows<false>, dim3(g2), dim3(256), 0, st, X, Xq, Xs, T, K, pos, k, shared_row0);
+    if (scatter && quant_rows_takes(K, k)) {
+        launch_quant_rows<false>(X, bf16, Xq, Xs, T, K, const_cast<int *>(pos), k, shared_row0, early, PlaceArgs{}, st);
     } else if (scatter) {
         if (bf16) launch_k(k_quant_e4m3<true, true>, dim3(grid), dim3(256), 0, st, X, Xq, Xs, T, K, pos, k, shared_row0);
         else launch_k(k_quant_e4m3<false, true>, dim3(grid), dim3(256), 0, st, X, Xq, Xs, T, K, pos, k, shared_row0);
@@ -786,7 +1032,7 @@ int launch_quant(const void *X, int bf16, uint8_t *Xq, uint8_t *Xs, int T, int K
 static constexpr int NOALLOC_MAX_ENTRIES = 16384;
 static constexpr int NOALLOC_MAX_EXPERTS = q36::DISPATCH_MAX_E;
 static constexpr size_t NOALLOC_SCRATCH_INTS =
-    (size_t)(NOALLOC_MAX_ENTRIES / q36::DISPATCH_CHUNK) * NOALLOC_MAX_EXPERTS + NOALLOC_MAX_ENTRIES;
+    (size_t)(NOALLOC_MAX_ENTRIES / q36::DISPATCH_CHUNK) * NOALLOC_MAX_EXPERTS + NOALLOC_MAX_ENTRIES / 2;
 static __device__ __align__(256) int g_noalloc_scratch[NOALLOC_SCRATCH_INTS];
 
 // Device address of the array above, looked up once per device.  In host code the symbol is only a
