@@ -134,4 +134,9 @@ int launch_ffn_fused_small(const void *Wg, const void *Wu, const void *Wd, const
                            const void *Sd, int n_group, int R_max, const uint8_t *Xq, const uint8_t *Xs, uint8_t *Hq,
                            uint8_t *Hs, float *Y, int D, int FF, void *plan, int *status, const EpReturnArgs *ep, cudaStream_t st);
 
+// moe_upload.cu: n_expert experts of `plane` 17-byte blocks each, from expert e0 on, into split planes on the device
+constexpr int UPLOAD_NOT_TAKEN = 1;
+int upload_repacked(const void *host_blocks, uint64_t plane, uint64_t e0, uint64_t n_expert, void *dev_dst);
+int upload_release();      // frees the pinned staging kept between uploads
+
 }  // namespace q36

@@ -202,15 +202,19 @@ int q36_moe_repack_mxfp4(const void *host_blocks, int K, int M, int e0, int e1, 
 }
 
 int q36_moe_upload_mxfp4(const void *host_blocks, int K, int M, int e0, int e1, void *dev_dst) {
-    if (!dev_dst) return Q36_MOE_EINVAL;
+    if (!dev_dst || !host_blocks || K < 0 || K % Q36_QK || M <= 0 || e0 < 0 || e1 <= e0) return Q36_MOE_EINVAL;
+    int rc = upload_repacked(host_blocks, (uint64_t)M * (K / Q36_QK), e0, e1 - e0, dev_dst);
+    if (rc != UPLOAD_NOT_TAKEN) return rc;
     const uint64_t bytes = (uint64_t)(e1 - e0) * q36_moe_expert_stride(M, K);
     void *tmp = malloc(bytes);
     if (!tmp) return Q36_MOE_ENOSPACE;
-    int rc = q36_moe_repack_mxfp4(host_blocks, K, M, e0, e1, tmp);
+    rc = q36_moe_repack_mxfp4(host_blocks, K, M, e0, e1, tmp);
     if (rc == Q36_MOE_OK) rc = ck(cudaMemcpy(dev_dst, tmp, bytes, cudaMemcpyHostToDevice));
     free(tmp);
     return rc;
 }
+
+int q36_moe_upload_release(void) { return upload_release(); }
 
 int q36_moe_dequant_mxfp4(const void *W, int M, int K, float *out, void *stream) {
     if (!W || !out || K % Q36_QK) return Q36_MOE_EINVAL;

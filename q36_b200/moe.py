@@ -39,6 +39,7 @@ _SIGS = {
     "q36_moe_expert_stride": (u64, [i32, i32]),
     "q36_moe_repack_mxfp4": (i32, [vp, i32, i32, i32, i32, vp]),
     "q36_moe_upload_mxfp4": (i32, [vp, i32, i32, i32, i32, vp]),
+    "q36_moe_upload_release": (i32, []),
     "q36_gguf_open": (i32, [C.c_char_p, C.POINTER(vp)]),
     "q36_gguf_close": (i32, [vp]),
     "q36_gguf_last_error": (C.c_char_p, []),
