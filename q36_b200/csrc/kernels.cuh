@@ -117,7 +117,8 @@ int make_map_codes(CUtensorMap *m, const void *base, int M, int K, int n_group, 
 int make_map_rows(CUtensorMap *m, const void *base, int R, int K, int box_rows);
 // the same planes seen as [.., K / 128 steps, rows, 128 elements] so that ONE copy fetches `ksteps` consecutive
 // K steps as consecutive 128-byte-swizzled tiles (coordinates: 0, row, K step [, expert])
-int make_map_codes_ksteps(CUtensorMap *m, const void *base, int M, int K, int n_group, uint64_t expert_stride, int ksteps);
+int make_map_codes_ksteps(CUtensorMap *m, const void *base, int M, int K, int n_group, uint64_t expert_stride, int ksteps,
+                          int box_rows = 128);
 int make_map_rows_ksteps(CUtensorMap *m, const void *base, int R, int K, int box_rows, int ksteps);
 int sm_count();            // of the CURRENT device
 int current_device();      // -1 when it cannot be determined or is beyond MAX_DEVICES

@@ -1168,11 +1168,11 @@ int make_map_codes(CUtensorMap *m, const void *base, int M, int K, int n_group, 
 // A thread needs ~140 cycles to issue any asynchronous copy, whatever its size, so the decode kernel fetches
 // several K steps per copy: the K axis is split into (step, 128 elements) and the step index becomes a box
 // dimension AFTER the rows, which lays the steps down as consecutive [rows][128 B] swizzled tiles.
-int make_map_codes_ksteps(CUtensorMap *m, const void *base, int M, int K, int n_group, uint64_t expert_stride, int ksteps) {
+int make_map_codes_ksteps(CUtensorMap *m, const void *base, int M, int K, int n_group, uint64_t expert_stride, int ksteps, int box_rows) {
     cuuint64_t dims[4] = {128, (cuuint64_t)M, (cuuint64_t)(K / 128), (cuuint64_t)n_group};
     cuuint64_t strides[3] = {(cuuint64_t)(K / 2), 64, (cuuint64_t)expert_stride};
-    cuuint32_t box[4] = {128, TC_M, (cuuint32_t)ksteps, 1};
-    return encode_cached(m, MapKey{base, expert_stride, 2, M, K, n_group, ksteps}, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 4, dims,
+    cuuint32_t box[4] = {128, (cuuint32_t)box_rows, (cuuint32_t)ksteps, 1};
+    return encode_cached(m, MapKey{base, expert_stride, 2, M, K, n_group, ksteps << 16 | box_rows}, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 4, dims,
                          strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 int make_map_rows_ksteps(CUtensorMap *m, const void *base, int R, int K, int box_rows, int ksteps) {

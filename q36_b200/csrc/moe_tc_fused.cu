@@ -35,21 +35,30 @@ namespace q36 {
 //    few extra down tiles (the lowest ranks: their inputs are there first) -- only as many as they can finish
 //    before the others join, since a group's rows arrive ~7000 cycles after its last gate/up MMA (epilogue,
 //    release fence, the polls); the rest is dealt round-robin;
+//  * with few groups a gate/up tile is 64 or 32 ff rows (RS = 2, 4; launch_ffn_fused_small has the rule): one token, 256
+//    experts: 26.7 us per layer before, 24.6 now;
 //  * a watcher thread walks the CTA's tile list ahead of everybody and, for a down tile, waits until the
 //    gate/up tiles of its group -- possibly on other SMs -- have published Hq/Hs; the other roles poll a
 //    count in shared memory, so that the L2 round trips of the check sit on nobody's issue path;
 //  * publishing costs a device-scope release fence, measured at ~2500 cycles under the weight stream: a
 //    publisher thread pays it, not the epilogue warps (they only signal through shared memory).
+// RS: a gate/up tile is 128 / RS ff rows (the plan counts 128-row tiles; this kernel cuts each into RS).  A stage then holds
+// four K steps of it; the MMA still takes 128 rows, of which the ones beyond the tile are whatever lies behind them in the
+// stage (an accumulator lane depends on its own row only, and nobody reads those lanes).
+template <int RS>
 struct FusedCfg {
-    static constexpr int STAGES = 4;
-    static constexpr int KS = 2;                     // K steps per stage
+    static constexpr int STAGES = 4;                 // even: a stage then always belongs to the same pair of issuers, which is
+                                                     // what makes their parity waits safe (nobody else follows its phases)
+    static constexpr int KS = 2;                     // K steps per stage of a down tile
+    static constexpr int KS_GU = RS == 1 ? 2 : 4;    // ... and of a gate/up tile
+    static constexpr int ROWS_GU = TC_M / RS;        // ff rows of a gate/up tile
     static constexpr int A_BYTES = TC_M * 128;       // one K step of one matrix, 4-bit codes in 8-bit containers
     static constexpr int A_TX_BYTES = TC_M * 64;     // the A box signals its packed bytes (see moe_tc.cu)
     static constexpr int B_BYTES = 16 * 128;
     static constexpr int SF_BYTES = 512;
-    static constexpr int OFF_B = KS * A_BYTES, OFF_SF = OFF_B + KS * B_BYTES;
-    static constexpr int STAGE_BYTES = OFF_SF + KS * 2 * SF_BYTES;          // 38 KB, 1024-aligned
-    static constexpr int STAGE_TX_A = KS * A_TX_BYTES, STAGE_TX_B = KS * B_BYTES;
+    static constexpr int OFF_B = KS * A_BYTES, OFF_SF = OFF_B + KS_GU * B_BYTES;
+    static constexpr int STAGE_BYTES = OFF_SF + KS_GU * 2 * SF_BYTES;       // 38 or 44 KB, 1024-aligned
+    static constexpr int TX_A_DN = KS * A_TX_BYTES, TX_A_GU = KS_GU * A_TX_BYTES / RS;
     // Scale bytes of a whole tile (all its K steps) are staged by bulk async copies, two tiles deep: the rows
     // of a tile are contiguous in the row-major scale planes (128 rows x K/32 bytes).  Loads issued by the
     // loader threads themselves were measured to expose a full HBM latency per 4 K steps (register prefetch
@@ -71,15 +80,16 @@ struct FusedCfg {
     static constexpr int MAX_GROUPS = DISPATCH_MAX_GROUPS + 1;   // the plan lists every group, empty ones included
     static constexpr int MAX_TILES = 192;                // per CTA
     static constexpr int TILE_ROWS = 16;                 // token rows per tile: the plan must be cut for this
-    static constexpr int EXTRA_DOWN = 3;                 // extra down tiles of a CTA that is one gate/up tile short
+    static constexpr int EXTRA_DOWN = 3 / RS;                 // extra down tiles of a CTA that is one gate/up tile short
 };
-static_assert(FusedCfg::STAGE_BYTES % 1024 == 0, "stage alignment");
+static_assert(FusedCfg<1>::STAGE_BYTES % 1024 == 0 && FusedCfg<2>::STAGE_BYTES % 1024 == 0 && FusedCfg<4>::STAGE_BYTES % 1024 == 0, "stage alignment");
 
 struct FusedMaps { CUtensorMap g, u, d, sg, su, sd, x, h; };
 
 struct FTile { int kind, g, mt, row0, nrows; };
 
-__global__ void __launch_bounds__(FusedCfg::THREADS, 1)
+template <int RS>
+__global__ void __launch_bounds__(FusedCfg<RS>::THREADS, 1)
 k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restrict__ sfG, const uint8_t *__restrict__ sfU,
                   const uint8_t *__restrict__ sfD, uint64_t sf_stride, const uint8_t *__restrict__ sfSG,
                   const uint8_t *__restrict__ sfSU, const uint8_t *__restrict__ sfSD, int n_routed,
@@ -89,7 +99,7 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
     // ep.peers != nullptr (the expert-parallel step): the result row of sorted row r < ep.n_map is the answer to the
     // received slot ep.rowmap[r] and goes straight into the result area of that slot's source rank, over NVLink,
     // instead of row r of Y; the last CTA to finish publishes the call's epoch in every source's header
-    using Cfg = FusedCfg;
+    using Cfg = FusedCfg<RS>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *sft = smem + Cfg::STAGES * Cfg::STAGE_BYTES;
@@ -138,8 +148,8 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
     // from here on: global memory written by earlier kernels (the plan, Xq/Xs)
 
     const int G = plan->n_groups;
-    const int n0 = plan->n_tiles[0], n_tiles = n0 + plan->n_tiles[1];
-    const int mt_gu = FF / TC_M;
+    const int n0 = plan->n_tiles[0] * RS, n_tiles = n0 + plan->n_tiles[1];
+    const int mt_gu = FF / Cfg::ROWS_GU;
     const int n1 = n_tiles - n0, grid = gridDim.x, b = blockIdx.x;
     // this CTA's list: its gate/up tiles, its extra down tiles if it is one gate/up tile short, its share of the rest
     const int n_long = n0 % grid;                              // CTAs [0, n_long) have one gate/up tile more
@@ -158,7 +168,7 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
         if (threadIdx.x == 0) atomicCAS(status, 0, 0x900);
     }
     for (int i = threadIdx.x; i <= G && fits; i += blockDim.x) {
-        s_base0[i] = plan->base[0][i];
+        s_base0[i] = plan->base[0][i] * RS;
         s_base1[i] = plan->base[1][i];
         if (i < G) { s_order[i] = (unsigned short)plan->order[i]; s_row0[i] = plan->row0[i]; s_cnt[i] = (unsigned short)plan->cnt[i]; }
     }
@@ -230,18 +240,19 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
                 const bool once = (int)s_cnt[t.g] <= Cfg::TILE_ROWS;    // a group of one token tile: its weights are read once
                 const CUtensorMap *ma0 = t.kind ? (sh ? &maps.sd : &maps.d) : (sh ? &maps.sg : &maps.g);
                 const CUtensorMap *ma1 = sh ? &maps.su : &maps.u;
-                const int nst = t.kind ? FF / (Cfg::KS * TC_KSTEP) : 2 * (D / (Cfg::KS * TC_KSTEP));   // gate, up, gate, ...
+                const int nst = t.kind ? FF / (Cfg::KS * TC_KSTEP) : 2 * (D / (Cfg::KS_GU * TC_KSTEP));   // gate, up, gate, ...
+                const int wrow0 = t.mt * (t.kind ? TC_M : Cfg::ROWS_GU), ksn = t.kind ? Cfg::KS : Cfg::KS_GU;
                 for (int q = 0; q < nst; q++, it++) {
                     const int kpair = t.kind ? q : (q >> 1);
                     const int s = it % Cfg::STAGES;
                     const uint32_t ph = (it / Cfg::STAGES) & 1;
                     if (!(ok = mbar_wait(empty0 + 8 * s, ph ^ 1, &abort_flag, status, 0x100 + s))) break;
                     const uint32_t sb = smem_u32(smem + s * Cfg::STAGE_BYTES);
-                    mbar_expect_tx(full0 + 8 * s, Cfg::STAGE_TX_A);
+                    mbar_expect_tx(full0 + 8 * s, t.kind ? Cfg::TX_A_DN : Cfg::TX_A_GU);
                     // weights that are read once per call: evict-first in L2, so that they do not displace the token rows,
                     // the intermediate and the scale bytes that other SMs re-read (measured: 25.95 against 26.5 us per launch)
-                    if (once) tma_load_4d_hint(sb, (!t.kind && (q & 1)) ? ma1 : ma0, 0, t.mt * TC_M, kpair * Cfg::KS, ge, full0 + 8 * s, w_policy);
-                    else tma_load_4d(sb, (!t.kind && (q & 1)) ? ma1 : ma0, 0, t.mt * TC_M, kpair * Cfg::KS, ge, full0 + 8 * s);
+                    if (once) tma_load_4d_hint(sb, (!t.kind && (q & 1)) ? ma1 : ma0, 0, wrow0, kpair * ksn, ge, full0 + 8 * s, w_policy);
+                    else tma_load_4d(sb, (!t.kind && (q & 1)) ? ma1 : ma0, 0, wrow0, kpair * ksn, ge, full0 + 8 * s);
                 }
             }
         }
@@ -260,8 +271,9 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
                 const uint32_t slot = j & 1;
                 if (!(ok = mbar_wait(sft_empty0 + 8 * slot, ((j >> 1) & 1) ^ 1, &abort_flag, status, 0x800 + slot))) break;
                 const int nbk = (t.kind ? FF : D) / Q36_QK;
-                const uint32_t a_bytes = TC_M * nbk, b_bytes = t.nrows * nbk;
-                const size_t arow = (size_t)ge * sf_stride + (size_t)(t.mt * TC_M) * nbk;
+                const int rows = t.kind ? TC_M : Cfg::ROWS_GU;
+                const uint32_t a_bytes = rows * nbk, b_bytes = t.nrows * nbk;
+                const size_t arow = (size_t)ge * sf_stride + (size_t)(t.mt * rows) * nbk;
                 const uint8_t *p0 = t.kind ? (sh ? sfSD : sfD) : (sh ? sfSG : sfG);
                 const uint32_t dst = smem_u32(sft + slot * Cfg::SFT_BYTES);
                 mbar_expect_tx(sft_full0 + 8 * slot, a_bytes * (t.kind ? 1 : 2) + b_bytes);
@@ -284,14 +296,15 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
                 const FTile t = get_tile(j);
                 if (t.kind) asm volatile("fence.proxy.async.global;" ::: "memory");   // as in the scale producer
                 const CUtensorMap *mb = t.kind ? &maps.h : &maps.x;
-                const int nst = t.kind ? FF / (Cfg::KS * TC_KSTEP) : 2 * (D / (Cfg::KS * TC_KSTEP));
+                const int ksn = t.kind ? Cfg::KS : Cfg::KS_GU;
+                const int nst = t.kind ? FF / (Cfg::KS * TC_KSTEP) : 2 * (D / (Cfg::KS_GU * TC_KSTEP));
                 for (int q = 0; q < nst; q++, it++) {
                     const int kpair = t.kind ? q : (q >> 1);
                     const int s = it % Cfg::STAGES;
                     const uint32_t ph = (it / Cfg::STAGES) & 1;
                     if (!(ok = mbar_wait(empty0 + 8 * s, ph ^ 1, &abort_flag, status, 0x180 + s))) break;
-                    mbar_expect_tx(full0 + 8 * s, Cfg::STAGE_TX_B);
-                    tma_load_3d(smem_u32(smem + s * Cfg::STAGE_BYTES) + Cfg::OFF_B, mb, 0, t.row0, kpair * Cfg::KS, full0 + 8 * s);
+                    mbar_expect_tx(full0 + 8 * s, ksn * Cfg::B_BYTES);
+                    tma_load_3d(smem_u32(smem + s * Cfg::STAGE_BYTES) + Cfg::OFF_B, mb, 0, t.row0, kpair * ksn, full0 + 8 * s);
                 }
             }
         }
@@ -299,13 +312,13 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
         // ----------------------------------------------------- MMA issuers
         if (lane == 0) {
             const int w = warp - Cfg::W_ISSUE0;
-            const int par = w >> 1, h = w & 1;             // stages with (stage & 1) == par, K step h of the stage
+            const int par = w >> 1, h = w & 1;             // stages with (stage & 1) == par, half h of the stage's K steps
             const uint32_t t_sfa = tmem + Cfg::SF_COL0 + 8 * w, t_sfb = t_sfa + 4;
             uint32_t it0 = 0;
             bool ok = true;
             for (int j = 0; j < my_tiles && ok; j++) {
                 const int kind = s_tiles[j].x >> 16;
-                const int nst = kind ? FF / (Cfg::KS * TC_KSTEP) : 2 * (D / (Cfg::KS * TC_KSTEP));
+                const int nst = kind ? FF / (Cfg::KS * TC_KSTEP) : 2 * (D / (Cfg::KS_GU * TC_KSTEP));
                 const uint32_t buf = j & 1;
                 const uint32_t d_tmem = tmem + buf * Cfg::ACC_STRIDE + 16 * w;
                 if (!(ok = mbar_wait(acc_empty0 + 8 * buf, ((j >> 1) & 1) ^ 1, &abort_flag, status, 0x200 + buf))) break;
@@ -318,17 +331,23 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
                     if (!(ok = mbar_wait(full0 + 8 * s, ph, &abort_flag, status, 0x300 + s))) break;
                     tc_fence_after();
                     const uint32_t sb = smem_u32(smem + s * Cfg::STAGE_BYTES);
-                    const uint32_t sa = sb + h * Cfg::A_BYTES, sbb = sb + Cfg::OFF_B + h * Cfg::B_BYTES;
-                    const uint32_t sf = sb + Cfg::OFF_SF + h * 2 * Cfg::SF_BYTES;
-                    tc_cp_sf(t_sfa, desc_sf(sf));
-                    tc_cp_sf(t_sfb, desc_sf(sf + Cfg::SF_BYTES));
+                    constexpr int HALF = Cfg::KS_GU / 2;
+                    const int k0 = kind ? h : h * HALF, k1 = kind ? h + 1 : (h + 1) * HALF;   // this issuer's half of the stage's K steps
+                    const uint32_t a_step = kind ? Cfg::A_BYTES : Cfg::A_BYTES / RS;
+#pragma unroll 1
+                    for (int ks = k0; ks < k1; ks++) {
+                        const uint32_t sa = sb + ks * a_step, sbb = sb + Cfg::OFF_B + ks * Cfg::B_BYTES;
+                        const uint32_t sf = sb + Cfg::OFF_SF + ks * 2 * Cfg::SF_BYTES;
+                        tc_cp_sf(t_sfa, desc_sf(sf));
+                        tc_cp_sf(t_sfb, desc_sf(sf + Cfg::SF_BYTES));
 #pragma unroll
-                    for (int kb = 0; kb < 4; kb++) {
-                        const uint32_t sfid = (uint32_t)kb << 30;
-                        tc_mma(d_tmem, desc_sw128(sa + kb * 32), desc_sw128(sbb + kb * 32), idesc_mx(16, kb),
-                               t_sfa | sfid, t_sfb | sfid, (first && kb == 0) ? 0u : 1u);
+                        for (int kb = 0; kb < 4; kb++) {
+                            const uint32_t sfid = (uint32_t)kb << 30;
+                            tc_mma(d_tmem, desc_sw128(sa + kb * 32), desc_sw128(sbb + kb * 32), idesc_mx(16, kb),
+                                   t_sfa | sfid, t_sfb | sfid, (first && kb == 0) ? 0u : 1u);
+                        }
+                        first = false;
                     }
-                    first = false;
                     tc_commit(empty0 + 8 * s);
                 }
                 it0 += nst;
@@ -345,7 +364,7 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
             const uint32_t tq = tmem + buf * Cfg::ACC_STRIDE + ((uint32_t)(q * 32) << 16);
             if (!(ok = mbar_wait(acc_full0 + 8 * buf, (j >> 1) & 1, &abort_flag, status, 0x400 + buf))) break;
             tc_fence_after();
-            const int mrow = t.mt * TC_M + q * 32 + lane;
+            const int mrow = t.mt * (t.kind ? TC_M : Cfg::ROWS_GU) + q * 32 + lane;
             // four partial sums of 16 token columns each (see FusedCfg)
             float g[16], u[16];
             {
@@ -365,7 +384,9 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
             if (lane == 0) mbar_arrive(acc_empty0 + 8 * buf);   // the registers hold the tile: TMEM is free again
             if (!t.kind) {
                 const int blk = mrow / Q36_QK;
-                if (t.nrows <= 2) {   // the usual routed group at decode: a short batch publishes sooner
+                if (q * 32 >= Cfg::ROWS_GU) {
+                    // (no rows of the tile in this lane quarter)
+                } else if (t.nrows <= 2) {   // the usual routed group at decode: a short batch publishes sooner
                     const float g0[2] = {g[0], g[1]}, u0[2] = {u[0], u[1]};
                     swiglu_quant_store<2>(g0, u0, t.nrows, (size_t)t.row0, Hq, Hs, FF, blk, lane);
                 } else {
@@ -458,28 +479,40 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
             const FTile t = get_tile(j);
             const uint32_t slot = j & 1;
             const int nbk = (t.kind ? FF : D) / Q36_QK;
-            const int nst = t.kind ? FF / (Cfg::KS * TC_KSTEP) : 2 * (D / (Cfg::KS * TC_KSTEP));
+            const int nst = t.kind ? FF / (Cfg::KS * TC_KSTEP) : 2 * (D / (Cfg::KS_GU * TC_KSTEP));
             if (!(ok = mbar_wait(sft_full0 + 8 * slot, (j >> 1) & 1, &abort_flag, status, 0x700 + slot))) break;
             const uint8_t *st = sft + slot * Cfg::SFT_BYTES;
             const uint8_t *ra0 = st + i * nbk, *ra1 = st + Cfg::SFT_A + i * nbk, *rb = st + 2 * Cfg::SFT_A + i * nbk;
             const bool bvalid = i < t.nrows;
-            for (int q0 = 0; q0 < nst && ok; q0 += 2) {   // two stages (four K steps) per cross-proxy fence
+            constexpr int QB = RS == 1 ? 2 : 1, NP = Cfg::KS_GU / 2;
+            const int ksn = t.kind ? Cfg::KS : Cfg::KS_GU;
+            for (int q0 = 0; q0 < nst && ok; q0 += QB) {   // four K steps of a gate/up tile per cross-proxy fence
                 const uint32_t it0 = it;
 #pragma unroll
-                for (int qq = 0; qq < 2; qq++) {
+                for (int qq = 0; qq < QB; qq++) {
                     const int q = q0 + qq;
                     const int kpair = t.kind ? q : (q >> 1);
                     const uint8_t *ra = (!t.kind && (q & 1)) ? ra1 : ra0;
-                    const uint2 va = *reinterpret_cast<const uint2 *>(ra + 8 * kpair);       // 2 K steps x 4 scale bytes
-                    const uint2 vb = bvalid ? *reinterpret_cast<const uint2 *>(rb + 8 * kpair) : make_uint2(0x7f7f7f7fu, 0x7f7f7f7fu);
+                    uint2 va[NP], vb[NP];                                                    // pairs of K steps x 4 scale bytes
+#pragma unroll
+                    for (int x = 0; x < NP; x++) {
+                        if (x > 0 && t.kind) break;
+                        va[x] = *reinterpret_cast<const uint2 *>(ra + 4 * ksn * kpair + 8 * x);
+                        vb[x] = bvalid ? *reinterpret_cast<const uint2 *>(rb + 4 * ksn * kpair + 8 * x) : make_uint2(0x7f7f7f7fu, 0x7f7f7f7fu);
+                    }
                     const int s = it % Cfg::STAGES;
                     const uint32_t ph = (it / Cfg::STAGES) & 1;
                     if (!(ok = mbar_wait(empty0 + 8 * s, ph ^ 1, &abort_flag, status, 0x500 + s))) break;
                     uint8_t *sf = smem + s * Cfg::STAGE_BYTES + Cfg::OFF_SF;
-                    *reinterpret_cast<uint32_t *>(sf + my_off) = va.x;
-                    *reinterpret_cast<uint32_t *>(sf + Cfg::SF_BYTES + my_off) = vb.x;
-                    *reinterpret_cast<uint32_t *>(sf + 2 * Cfg::SF_BYTES + my_off) = va.y;
-                    *reinterpret_cast<uint32_t *>(sf + 3 * Cfg::SF_BYTES + my_off) = vb.y;
+#pragma unroll
+                    for (int x = 0; x < NP; x++) {
+                        if (x > 0 && t.kind) break;
+                        uint8_t *im = sf + x * 4 * Cfg::SF_BYTES + my_off;
+                        *reinterpret_cast<uint32_t *>(im) = va[x].x;
+                        *reinterpret_cast<uint32_t *>(im + Cfg::SF_BYTES) = vb[x].x;
+                        *reinterpret_cast<uint32_t *>(im + 2 * Cfg::SF_BYTES) = va[x].y;
+                        *reinterpret_cast<uint32_t *>(im + 3 * Cfg::SF_BYTES) = vb[x].y;
+                    }
                     it++;
                 }
                 if (!ok) break;
@@ -523,7 +556,7 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
 // Does the per-CTA tile table hold a call of R_max rows in n_group (+ 1 shared) groups?  A group of c rows is
 // ceil(c / 16) token tiles, so there are at most R_max / 16 + (non-empty groups) of them.
 bool ffn_fused_small_fits(int R_max, int n_group, int D, int FF) {
-    using Cfg = FusedCfg;
+    using Cfg = FusedCfg<1>;
     // the staged scale bytes of a tile are sized for K <= K_MAX; larger layers take the two grouped-GEMM launches
     if (D > Cfg::K_MAX || FF > Cfg::K_MAX || D % (4 * TC_KSTEP) || FF % (4 * TC_KSTEP)) return false;
     const long tt = R_max / Cfg::TILE_ROWS + min(R_max, n_group + 1);
@@ -537,32 +570,48 @@ int ffn_fused_small_grid(int R_max, int n_group, int D, int FF) {
     return (int)min((long)sm_count(), max_tiles);
 }
 
-int launch_ffn_fused_small(const void *Wg, const void *Wu, const void *Wd, const void *Sg, const void *Su,
-                           const void *Sd, int n_group, int R_max, const uint8_t *Xq, const uint8_t *Xs, uint8_t *Hq,
-                           uint8_t *Hs, float *Y, int D, int FF, void *plan, int *status, const EpReturnArgs *ep, cudaStream_t st) {
-    using Cfg = FusedCfg;
-    if (D % (4 * TC_KSTEP) || FF % (4 * TC_KSTEP) || !ffn_fused_small_fits(R_max, n_group, D, FF)) return Q36_MOE_EINVAL;
+template <int RS>
+static int run_ffn_fused(const void *Wg, const void *Wu, const void *Wd, const void *Sg, const void *Su, const void *Sd, int n_group, int R_max,
+                         const uint8_t *Xq, const uint8_t *Xs, uint8_t *Hq, uint8_t *Hs, float *Y, int D, int FF, void *plan, int *status,
+                         const EpReturnArgs *ep, cudaStream_t st) {
+    using Cfg = FusedCfg<RS>;
     const uint64_t estride = (uint64_t)FF * (D / 2) + (uint64_t)FF * (D / Q36_QK);   // same for [FF][D] and [D][FF]
     const uint64_t plane = (uint64_t)FF * (D / 2);
     if (!Sg) { Sg = Wg; Su = Wu; Sd = Wd; }
     FusedMaps maps;
     int rc;
-    if ((rc = make_map_codes_ksteps(&maps.g, Wg, FF, D, n_group, estride, Cfg::KS))) return rc;
-    if ((rc = make_map_codes_ksteps(&maps.u, Wu, FF, D, n_group, estride, Cfg::KS))) return rc;
+    if ((rc = make_map_codes_ksteps(&maps.g, Wg, FF, D, n_group, estride, Cfg::KS_GU, Cfg::ROWS_GU))) return rc;
+    if ((rc = make_map_codes_ksteps(&maps.u, Wu, FF, D, n_group, estride, Cfg::KS_GU, Cfg::ROWS_GU))) return rc;
     if ((rc = make_map_codes_ksteps(&maps.d, Wd, D, FF, n_group, estride, Cfg::KS))) return rc;
-    if ((rc = make_map_codes_ksteps(&maps.sg, Sg, FF, D, 1, estride, Cfg::KS))) return rc;
-    if ((rc = make_map_codes_ksteps(&maps.su, Su, FF, D, 1, estride, Cfg::KS))) return rc;
+    if ((rc = make_map_codes_ksteps(&maps.sg, Sg, FF, D, 1, estride, Cfg::KS_GU, Cfg::ROWS_GU))) return rc;
+    if ((rc = make_map_codes_ksteps(&maps.su, Su, FF, D, 1, estride, Cfg::KS_GU, Cfg::ROWS_GU))) return rc;
     if ((rc = make_map_codes_ksteps(&maps.sd, Sd, D, FF, 1, estride, Cfg::KS))) return rc;
-    if ((rc = make_map_rows_ksteps(&maps.x, Xq, R_max, D, 16, Cfg::KS))) return rc;
+    if ((rc = make_map_rows_ksteps(&maps.x, Xq, R_max, D, 16, Cfg::KS_GU))) return rc;
     if ((rc = make_map_rows_ksteps(&maps.h, Hq, R_max, FF, 16, Cfg::KS))) return rc;
-    static bool attr_done[MAX_DEVICES] = {false};
-    if ((rc = ensure_smem_attr((const void *)k_ffn_fused_small, Cfg::SMEM_BYTES, attr_done))) return rc;
+    static bool attr_done[MAX_DEVICES] = {false};   // one array per instantiation
+    if ((rc = ensure_smem_attr((const void *)k_ffn_fused_small<RS>, Cfg::SMEM_BYTES, attr_done))) return rc;
     const int grid = ffn_fused_small_grid(R_max, n_group, D, FF);
-    launch_k_resident(k_ffn_fused_small, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, st, maps, (const uint8_t *)Wg + plane,
+    launch_k_resident(k_ffn_fused_small<RS>, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, st, maps, (const uint8_t *)Wg + plane,
              (const uint8_t *)Wu + plane, (const uint8_t *)Wd + plane, estride, (const uint8_t *)Sg + plane,
              (const uint8_t *)Su + plane, (const uint8_t *)Sd + plane, n_group, Xs, (TcPlan *)plan, Hq, Hs, Y, D, FF, status,
              ep ? *ep : EpReturnArgs{nullptr, 0, 0, 0, 0, nullptr, nullptr, 0, 0, 0, 0, 0});
     return check_launch();
+}
+
+int launch_ffn_fused_small(const void *Wg, const void *Wu, const void *Wd, const void *Sg, const void *Su,
+                           const void *Sd, int n_group, int R_max, const uint8_t *Xq, const uint8_t *Xs, uint8_t *Hq,
+                           uint8_t *Hs, float *Y, int D, int FF, void *plan, int *status, const EpReturnArgs *ep, cudaStream_t st) {
+    if (D % (4 * TC_KSTEP) || FF % (4 * TC_KSTEP) || !ffn_fused_small_fits(R_max, n_group, D, FF)) return Q36_MOE_EINVAL;
+    // Few groups leave most SMs without a gate/up tile of 128 rows: 9 groups (one token, 8 + 1 experts) are 36 tiles on 148
+    // SMs, each 280 KB for one SM to fetch.  Tiles are cut as long as the pieces still fit in one round; beyond that a
+    // shorter tile only costs (the MMAs and token rows of a tile are the same for any height).  40 layers, us per pass with
+    // tiles of 128 / 64 / 32 rows: 9 groups 1068 / 987 / 983, 13 groups 997 / 954 / 1064, 57 groups 1393 / 1464 / 1916; 16
+    // layers of 41 groups 706 / 707 / 829.
+    const int groups = min(R_max, n_group + 1);
+    const long tiles = (groups + (long)(R_max - groups) / FusedCfg<1>::TILE_ROWS) * (FF / TC_M);   // (an upper bound)
+    const int rs = ep ? 1 : tiles * 4 <= sm_count() ? 4 : tiles * 2 <= sm_count() ? 2 : 1;
+    auto run = rs == 4 ? run_ffn_fused<4> : rs == 2 ? run_ffn_fused<2> : run_ffn_fused<1>;
+    return run(Wg, Wu, Wd, Sg, Su, Sd, n_group, R_max, Xq, Xs, Hq, Hs, Y, D, FF, plan, status, ep, st);
 }
 
 }  // namespace q36

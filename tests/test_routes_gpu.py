@@ -53,3 +53,21 @@ def test_uploads_from_several_threads_do_not_disturb_each_other(moe):
         want = np.empty(g.numel(), np.uint8)
         moe.check(moe.lib.q36_moe_repack_mxfp4(b.ctypes.data, 2048, 1024, 0, 3, want.ctypes.data), "repack")
         np.testing.assert_array_equal(g.cpu().numpy(), want)
+
+
+# gate/up tiles of 32 ff rows while the groups' tiles are at most the SMs (148: 9 groups x 16), 64 up to 18 groups, then 128
+@pytest.mark.parametrize("k,T,se0,se1,shared", [(4, 1, 0, 32, True), (8, 1, 0, 32, True), (8, 1, 0, 32, False), (4, 2, 0, 32, True),
+                                                (2, 3, 0, 32, True), (4, 3, 0, 32, True), (8, 2, 0, 32, True), (4, 4, 0, 32, True),
+                                                (8, 3, 0, 32, True), (8, 16, 8, 16, False), (8, 16, 8, 24, False), (8, 40, 0, 8, True),
+                                                (4, 100, 24, 32, False)])
+def test_gateup_tile_heights_agree_with_the_cuda_core_path(moe, k, T, se0, se1, shared):
+    import torch
+    ly = moe.MoELayer(n_expert=32, k=k, se0=se0, se1=se1).random_planes(3 + k, shared=shared)
+    rng = np.random.default_rng(10 * T + k)
+    X = torch.from_numpy(synth.activations(rng, T)).cuda().to(torch.bfloat16)
+    L = torch.from_numpy(synth.router_logits(rng, T, 32)).cuda()
+    a = ly.forward(X, L, path=moe.PATH_TC, inc_shared=shared)
+    ly.check_device_status()
+    b = ly.forward(X, L, path=moe.PATH_GEMV, inc_shared=shared)
+    # f32 sums in another order; a value of the E4M3 intermediate on a rounding boundary may fall on its other side (1e-3 of its row)
+    assert float(b.abs().max()) > 0 and rel_l2(a, b) < 2e-3
