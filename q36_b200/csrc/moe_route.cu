@@ -805,7 +805,8 @@ k_front_decode(const float *__restrict__ logits, int n_expert, int k, float scal
         if (e >= 0 && r_in_warp == 0) cnt[warp][e] = (unsigned short)__popc(peers);
     }
     __syncthreads();
-    // per expert: rows, and (one scan for both) rows before it | non-empty experts before it << 16
+    // per expert: rows, and (one scan for both) rows before it | token tiles of 16 rows before it << 16 (16 tokens with several
+    // entries of one expert each, as rows with fewer than k eligible logits have, are more than one tile)
     int tot = 0;
     if (tid < n_expert) {
         for (int w = 0; w < used_warps; w++) {
@@ -814,7 +815,7 @@ k_front_decode(const float *__restrict__ logits, int n_expert, int k, float scal
             tot += c;
         }
     }
-    const int val = tot | ((tot > 0) << 16);
+    const int val = tot | ((tot + 15) / 16 << 16);
     int incl = val;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += u; }

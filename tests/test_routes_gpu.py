@@ -71,3 +71,19 @@ def test_gateup_tile_heights_agree_with_the_cuda_core_path(moe, k, T, se0, se1, 
     b = ly.forward(X, L, path=moe.PATH_GEMV, inc_shared=shared)
     # f32 sums in another order; a value of the E4M3 intermediate on a rounding boundary may fall on its other side (1e-3 of its row)
     assert float(b.abs().max()) > 0 and rel_l2(a, b) < 2e-3
+
+
+def test_decode_rows_with_one_eligible_expert(moe):
+    """Rows whose other logits are masked out fill their remaining slots with expert 0 at weight 0: 16 tokens then have 112
+    entries of that expert, more than one 16-row token tile."""
+    import torch
+    E, k, T = 32, 8, 16
+    L = torch.full((T, E + 1), float("-inf"), device="cuda")
+    L[torch.arange(T), 1 + torch.arange(T)] = 1.0
+    L[:, E] = 0.5
+    ly = moe.MoELayer(n_expert=E, k=k).random_planes(2)
+    X = torch.from_numpy(synth.activations(np.random.default_rng(2), T)).cuda().to(torch.bfloat16)
+    out = ly.forward(X, L)
+    ly.check_device_status()
+    want = ly.forward(X, L, path=moe.PATH_GEMV)
+    assert bool(torch.isfinite(want).all()) and rel_l2(out, want) < 2e-3
