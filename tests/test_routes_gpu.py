@@ -73,6 +73,68 @@ def test_gateup_tile_heights_agree_with_the_cuda_core_path(moe, k, T, se0, se1, 
     assert float(b.abs().max()) > 0 and rel_l2(a, b) < 2e-3
 
 
+# cluster front end up to 512 tokens (at k = 8), two launches beyond; the decode cluster up to 16
+@pytest.mark.parametrize("E,k", [(256, 8), (128, 6), (64, 1), (32, 8)])
+@pytest.mark.parametrize("T", [16, 17, 63, 64, 65, 511, 512, 513, 1025])
+def test_front_end_of_any_batch(moe, oracle, E, k, T):
+    import torch
+    rng = np.random.default_rng(T + E)
+    L = synth.router_logits(rng, T, E, zipf=T % 2 == 1)
+    L[T // 2, : E // 2] = 0.25                               # ties: the lower id wins
+    ly = moe.MoELayer(n_expert=E, k=k).random_planes(E)
+    X = torch.from_numpy(synth.activations(rng, T)).cuda().to(torch.bfloat16)
+    lt = torch.from_numpy(L).cuda()
+    out, idx, wt = ly.forward(X, lt, want_routing=True)
+    ly.check_device_status()
+    sidx, swt = moe.router_topk(lt, E, k)                    # the router entry on its own
+    assert torch.equal(idx, sidx) and torch.equal(wt, swt)
+    widx, _ = oracle.router_topk(L, k, n_expert=E)
+    np.testing.assert_array_equal(idx.cpu().numpy(), widx)
+    want = ly.forward(X, lt, path=moe.PATH_GEMV)
+    assert rel_l2(out, want) < 2e-3                          # as above
+
+
+def test_router_rows_without_a_largest_value(moe):
+    """NaN, infinities and the lowest values: every route must choose what the router entry chooses."""
+    import torch
+    E, k = 64, 4
+    low = torch.finfo(torch.float32).min
+    for T in (8, 40, 600):
+        g = torch.Generator(device="cuda")
+        g.manual_seed(T)
+        L = torch.randn((T, E + 1), device="cuda", generator=g)
+        L[0, :E] = float("-inf")
+        L[1, :E] = low
+        L[2, 3] = float("nan")
+        L[3, 5:] = float("-inf")
+        L[4, 7] = float("inf")
+        L[5, 2:] = low                                       # two experts to choose from, four wanted
+        ly = moe.MoELayer(n_expert=E, k=k).random_planes(1)
+        X = torch.randn((T, D), device="cuda", generator=g)
+        _, idx, wt = ly.forward(X, L, want_routing=True)
+        ly.check_device_status()
+        sidx, swt = moe.router_topk(L, E, k)
+        assert torch.equal(idx, sidx) and torch.equal(wt.isnan(), swt.isnan())
+        assert torch.equal(wt.nan_to_num(), swt.nan_to_num())
+        assert int(idx.min()) >= 0 and int(idx.max()) < E
+
+
+# the logits kernels: rows in registers (1, 2, 4, 8, 16 tokens), then 32-, 64- and 128-token tiles with K split 8, 4 or 1 ways
+@pytest.mark.parametrize("T,n_rows", [(1, 33), (2, 257), (3, 65), (5, 257), (9, 129), (16, 257), (17, 257), (33, 33), (128, 257), (129, 129),
+                                      (1000, 257), (1025, 257), (4097, 33), (20000, 257)])
+def test_router_logits_at_the_changes_of_tile(moe, T, n_rows):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(T)
+    h = torch.randn((T, D), device="cuda", generator=g)
+    w = 1 + 0.1 * torch.randn(D, device="cuda", generator=g)
+    router = torch.randn((n_rows, D), device="cuda", generator=g) / D ** 0.5
+    x, logits = moe.pre_norm_router(h, None, w, router, gate_row=n_rows - 1)
+    want = x.double() @ router.double().T
+    # sums of 2048 f32 products whose partial sums stay below a few units: far below 2048 ulps of the largest
+    assert float((logits.double() - want).abs().max()) < 2e-5 * float(want.abs().max())
+
+
 def test_decode_rows_with_one_eligible_expert(moe):
     """Rows whose other logits are masked out fill their remaining slots with expert 0 at weight 0: 16 tokens then have 112
     entries of that expert, more than one 16-row token tile."""
