@@ -305,7 +305,7 @@ k_combine_add_rmsnorm(float *__restrict__ moe_out, const float *__restrict__ Y, 
             m.z = fmaf(wgt[s], y[s].z, m.z); m.w = fmaf(wgt[s], y[s].w, m.w);
         }
         if (SH) { m.x = fmaf(gs, ysh.x, m.x); m.y = fmaf(gs, ysh.y, m.y); m.z = fmaf(gs, ysh.z, m.z); m.w = fmaf(gs, ysh.w, m.w); }
-        if (moe_out) reinterpret_cast<float4 *>(moe_out + (size_t)t * D)[i] = m;
+        if (moe_out) __stcs(reinterpret_cast<float4 *>(moe_out + (size_t)t * D) + i, m);
         float4 r = make_float4(hv.x + m.x, hv.y + m.y, hv.z + m.z, hv.w + m.w);
         reinterpret_cast<float4 *>(h + (size_t)t * D)[i] = r;
         acc[j] = r;

@@ -247,7 +247,7 @@ k_combine(float *__restrict__ out, const float *__restrict__ Y, const int *__res
         acc.x = fmaf(gs, ysh.x, acc.x); acc.y = fmaf(gs, ysh.y, acc.y);
         acc.z = fmaf(gs, ysh.z, acc.z); acc.w = fmaf(gs, ysh.w, acc.w);
     }
-    *reinterpret_cast<float4 *>(out + (size_t)t * D + i) = acc;
+    __stcs(reinterpret_cast<float4 *>(out + (size_t)t * D + i), acc);
 }
 
 // dst row i = src row index[i] (16-byte units); negative index -> zeros
