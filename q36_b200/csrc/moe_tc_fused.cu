@@ -312,7 +312,7 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
         // ----------------------------------------------------- MMA issuers
         if (lane == 0) {
             const int w = warp - Cfg::W_ISSUE0;
-            const int par = w >> 1, h = w & 1;             // stages with (stage & 1) == par, half h of the stage's K steps
+            const int par = w >> 1, h = w & 1;             // stages with (stage & 1) == par, the stage's K steps h, h + 2, ...
             const uint32_t t_sfa = tmem + Cfg::SF_COL0 + 8 * w, t_sfb = t_sfa + 4;
             uint32_t it0 = 0;
             bool ok = true;
@@ -331,11 +331,12 @@ k_ffn_fused_small(const __grid_constant__ FusedMaps maps, const uint8_t *__restr
                     if (!(ok = mbar_wait(full0 + 8 * s, ph, &abort_flag, status, 0x300 + s))) break;
                     tc_fence_after();
                     const uint32_t sb = smem_u32(smem + s * Cfg::STAGE_BYTES);
-                    constexpr int HALF = Cfg::KS_GU / 2;
-                    const int k0 = kind ? h : h * HALF, k1 = kind ? h + 1 : (h + 1) * HALF;   // this issuer's half of the stage's K steps
+                    const int ksn = kind ? Cfg::KS : Cfg::KS_GU;
                     const uint32_t a_step = kind ? Cfg::A_BYTES : Cfg::A_BYTES / RS;
+                    // every other K step: an accumulator sums the same K steps in the same order at every tile height, so that
+                    // a token's result does not depend on how many tokens share its call
 #pragma unroll 1
-                    for (int ks = k0; ks < k1; ks++) {
+                    for (int ks = h; ks < ksn; ks += 2) {
                         const uint32_t sa = sb + ks * a_step, sbb = sb + Cfg::OFF_B + ks * Cfg::B_BYTES;
                         const uint32_t sf = sb + Cfg::OFF_SF + ks * 2 * Cfg::SF_BYTES;
                         tc_cp_sf(t_sfa, desc_sf(sf));

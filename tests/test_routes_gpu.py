@@ -73,6 +73,22 @@ def test_gateup_tile_heights_agree_with_the_cuda_core_path(moe, k, T, se0, se1, 
     assert float(b.abs().max()) > 0 and rel_l2(a, b) < 2e-3
 
 
+def test_gateup_tile_heights_give_the_same_bits(moe):
+    """A token's result does not depend on the tile height: calls of one token (9 groups: tiles of 32 ff rows), two (18: 64 rows)
+    and all sixteen (128 rows) sum the same products in the same order."""
+    import torch
+    T = 16
+    ly = moe.MoELayer(n_expert=64, k=8).random_planes(5)
+    rng = np.random.default_rng(5)
+    X = torch.from_numpy(synth.activations(rng, T)).cuda().to(torch.bfloat16)
+    L = torch.from_numpy(synth.router_logits(rng, T, 64)).cuda()
+    want = ly.forward(X, L)
+    for n in (1, 2):
+        got = torch.cat([ly.forward(X[t:t + n].contiguous(), L[t:t + n].contiguous()) for t in range(0, T, n)])
+        ly.check_device_status()
+        assert torch.equal(got, want), f"{n} token(s) per call"
+
+
 # cluster front end up to 512 tokens (at k = 8), two launches beyond; the decode cluster up to 16
 @pytest.mark.parametrize("E,k", [(256, 8), (128, 6), (64, 1), (32, 8)])
 @pytest.mark.parametrize("T", [16, 17, 63, 64, 65, 511, 512, 513, 1025])
