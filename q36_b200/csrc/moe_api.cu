@@ -112,8 +112,9 @@ static int layer_impl(const void *Wg, const void *Wu, const void *Wd, const void
     // decode: gate/up and down in one persistent launch (its plan is cut in token tiles of 16 rows)
     const bool decode_kernel = use_tc && !no_fuse && R <= fused_rows_limit() && ffn_fused_small_fits(R, se1 - se0, D, FF);
     static const bool no_cluster = getenv("Q36_NOCLUSTER") != nullptr;
-    // decode on the tensor-core path with every expert resident: one cluster launch does all of the front end
-    const bool cluster_front = use_tc && T <= 16 && n <= 128 && se0 == 0 && se1 == E && D % 1024 == 0 && D * T <= 32 * 1024 && !no_cluster;
+    // in front of the decode kernel, with every expert resident: one cluster launch does all of the front end (it lays its plan
+    // for that kernel's 16-row token tiles, which the grouped-GEMM launches of other shapes do not take)
+    const bool cluster_front = decode_kernel && T <= 16 && n <= 128 && se0 == 0 && se1 == E && D % 1024 == 0 && D * T <= 32 * 1024 && !no_cluster;
     const int plan_rows = decode_kernel ? 16 : gateup_tile_rows(), sh0 = n, sh1 = shared ? n + T : n;
     if (cluster_front) {
         if ((rc = launch_front_decode(logits, E, k, route_scale, T, logit_stride, w.idx, w.wt, w.ecount, w.eoffs, w.elist,

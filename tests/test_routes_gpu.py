@@ -165,3 +165,24 @@ def test_decode_rows_with_one_eligible_expert(moe):
     ly.check_device_status()
     want = ly.forward(X, L, path=moe.PATH_GEMV)
     assert bool(torch.isfinite(want).all()) and rel_l2(out, want) < 2e-3
+
+
+# hidden 4096 is beyond the decode kernel: the grouped-GEMM launches follow the front end at every batch, and need its plan in their
+# own token tiles; with one eligible expert per row 56 of the 64 rows fall to expert 0
+@pytest.mark.parametrize("T,masked", [(1, False), (8, False), (8, True), (9, False)])
+def test_decode_batches_of_a_layer_the_decode_kernel_does_not_take(moe, T, masked):
+    import torch
+    E, k, D4 = 32, 8, 4096
+    assert not moe.lib.q36_moe_one_launch_fits(T * (k + 1), E, D4, FF)
+    ly = moe.MoELayer(n_expert=E, k=k, D=D4).random_planes(4)
+    rng = np.random.default_rng(T)
+    X = torch.from_numpy(synth.activations(rng, T, D4)).cuda().to(torch.bfloat16)
+    L = torch.from_numpy(synth.router_logits(rng, T, E)).cuda()
+    if masked:
+        L[:, :E] = float("-inf")
+        L[torch.arange(T), 1 + torch.arange(T)] = 1.0
+    out = ly.forward(X, L)
+    ly.check_device_status()
+    want = ly.forward(X, L, path=moe.PATH_GEMV)
+    # f32 sums in another order; E4M3 values of the intermediate on a rounding boundary (1e-3 of a row)
+    assert bool(torch.isfinite(want).all()) and float(want.abs().max()) > 0 and rel_l2(out, want) < 2e-3
