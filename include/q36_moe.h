@@ -72,7 +72,8 @@ int q36_moe_repack_mxfp4(const void *host_blocks, int K, int M, int e0, int e1, 
 /* Host -> device: same, then copies into the caller's device buffer dev_dst
  * of (e1-e0)*q36_moe_expert_stride(M,K) bytes.  Synchronous, like upload(). */
 int q36_moe_upload_mxfp4(const void *host_blocks, int K, int M, int e0, int e1, void *dev_dst);
-/* Uploads keep up to 8.5 MB of pinned host memory for the next one; this gives it back (when the model is loaded). */
+/* Uploads keep up to 8.5 MB of pinned host memory and, per device, eight streams for the next one; this gives them back
+ * (when the model is loaded). */
 int q36_moe_upload_release(void);
 /* Device: split planes -> f32 [n_rows][K] (row r of the expert at W).  The
  * on-device form of q36_deq_row(Q36_GGML_MXFP4, ...) (q36_dequant.cuh:168-181),

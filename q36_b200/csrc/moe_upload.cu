@@ -6,6 +6,7 @@
 // second host copy, no device staging, and the threads' copies overlap the transfer.  What bounds it is then the PCIe
 // link and the host's copy into pinned memory.  A layer of 64 + 1 experts (109 MB, six uploads): 4.7 ms; 47.6 when one
 // host thread took the blocks apart and a pageable copy followed; 45 when every upload pinned its own staging.
+#include <cuda.h>
 #include <string.h>
 
 #include <atomic>
@@ -29,8 +30,7 @@ static_assert(RP_BLOCKS * 17 % 16 == 0 && UP_SLOT_BYTES % 16 == 0, "16-byte load
 // `first` of the tensor; plane: blocks per expert.  dst and the experts' stride (plane * 17) are multiples of 16 bytes.
 __global__ void __launch_bounds__(RP_BLOCKS)
 k_repack(const uint4 *__restrict__ src, uint64_t first, int n, uint64_t plane, uint8_t *__restrict__ dst) {
-    // the next slot's kernel has nothing to do with this one: let its reads start behind this one's
-    cudaTriggerProgrammaticLaunchCompletion();
+    Q36_GDS();
     __shared__ uint4 s4[RP_BLOCKS * 17 / 16 + 1];       // (+ 1: the last block's shifted reads touch one word more)
     const int b0 = blockIdx.x * RP_BLOCKS, nb = min(RP_BLOCKS, n - b0);
     const int words = (nb * 17 + 15) / 16;
@@ -47,12 +47,18 @@ k_repack(const uint4 *__restrict__ src, uint64_t first, int n, uint64_t plane, u
     codes[plane * 16 + r] = reinterpret_cast<const uint8_t *>(s4)[threadIdx.x * 17];
 }
 
+// A slot's transfer takes 10 us and a kernel's start and end 6 more, so kernels have to overlap.  Every thread has a stream of
+// its own for that: "the slot's kernel is over" is then one event, whatever the others do.  One stream with overlapping kernels
+// would need each of them to wait for the one before it before it ends, else the end of one says nothing about the ones before:
+// that chain leaves two kernels in flight.  Loads of 64 + 1 experts with 8 streams 3.8 ms, 4 streams 4.4, 2 streams 4.7; one
+// stream 5.8 (kernels in turn) or 5.3 (overlapping, with the wait).
+//
 // Pinned staging.  Pinning costs more than the transfer (4 to 10 ms for the 8.5 MB of one upload, which takes 1.5), so one
 // staging area of at most that size stays with the process between uploads; q36_moe_upload_release gives it back.  An upload
 // that finds it in use by another thread pins and frees its own.
 namespace {
 struct Staging { uint8_t *p; uint64_t bytes; };
-std::mutex g_staging_mutex;
+std::mutex g_staging_mutex;                             // (also of g_lanes)
 Staging g_staging = {nullptr, 0};
 
 Staging staging_swap(Staging s, bool only_larger) {
@@ -82,23 +88,79 @@ cudaError_t staging_put(Staging s) {
     s = staging_swap(s, true);                          // keep the larger one
     return s.p ? cudaFreeHost(s.p) : cudaSuccess;
 }
+
+// The threads' streams stay as well: making one and destroying it costs 120 us, as much as a small upload.  One set per device,
+// of the context it was made in; an upload that finds it in use makes and destroys its own.
+struct Lanes { unsigned long long ctx; cudaStream_t st[UP_MAX_THREADS]; };
+Lanes g_lanes[MAX_DEVICES] = {};
+
+void *driver_fn(const char *name) {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? p : nullptr;
+}
+// id of the calling thread's context (no two contexts of a process have the same one), 0 if it cannot be had
+unsigned long long context_id() {
+    static const auto get = (CUresult (*)(CUcontext *))driver_fn("cuCtxGetCurrent");
+    static const auto get_id = (CUresult (*)(CUcontext, unsigned long long *))driver_fn("cuCtxGetId");
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (!get || !get_id || get(&c) != CUDA_SUCCESS || !c || get_id(c, &id) != CUDA_SUCCESS) return 0;
+    return id;
+}
+Lanes lanes_take(int dev, unsigned long long ctx) {
+    Lanes l = {};
+    {
+        std::lock_guard<std::mutex> lock(g_staging_mutex);
+        std::swap(l, g_lanes[dev]);
+    }
+    if (l.ctx != ctx) l = Lanes{ctx, {}};               // (another context's streams went, or go, with it)
+    return l;
+}
+cudaError_t lanes_put(int dev, Lanes l, bool keep) {
+    if (keep) {
+        std::lock_guard<std::mutex> lock(g_staging_mutex);
+        if (!g_lanes[dev].ctx) std::swap(l, g_lanes[dev]);
+    }
+    cudaError_t e = cudaSuccess;
+    for (cudaStream_t st : l.st)
+        if (st) { const cudaError_t d = cudaStreamDestroy(st); if (e == cudaSuccess) e = d; }
+    return e;
+}
 }  // namespace
 
 int upload_release() {
+    cudaError_t el = cudaSuccess;
+    int cur = -1;
+    if (cudaGetDevice(&cur) != cudaSuccess) (void)cudaGetLastError();
+    for (int dev = 0; dev < MAX_DEVICES; dev++) {
+        bool any;
+        {
+            std::lock_guard<std::mutex> lock(g_staging_mutex);
+            any = g_lanes[dev].ctx != 0;
+        }
+        if (!any || (dev != cur && cudaSetDevice(dev) != cudaSuccess)) continue;
+        const cudaError_t e = lanes_put(dev, lanes_take(dev, context_id()), false);
+        if (el == cudaSuccess) el = e;
+        if (dev != cur && cur >= 0) (void)cudaSetDevice(cur);
+    }
     const Staging s = staging_swap(Staging{nullptr, 0}, false);
-    const cudaError_t e = staging_alive(s) ? cudaFreeHost(s.p) : cudaSuccess;
+    cudaError_t e = staging_alive(s) ? cudaFreeHost(s.p) : cudaSuccess;
+    if (e == cudaSuccess) e = el;
     if (e != cudaSuccess) { last_cuda_error() = (int)e; return Q36_MOE_ECUDA; }
     return Q36_MOE_OK;
 }
 
 // Returns UPLOAD_NOT_TAKEN when this route does not apply (see the rule) or pinned memory cannot be had; the caller then
-// re-arranges on the host.  Synchronous, ordered like a cudaMemcpy: everything is issued on the legacy default stream.
+// re-arranges on the host.  Synchronous, ordered like a cudaMemcpy: the first byte's copy waits for
+// what the legacy default stream would wait for, and the threads' streams wait for that stream.
 int upload_repacked(const void *host_blocks, uint64_t plane, uint64_t e0, uint64_t n_expert, void *dev_dst) {
     // 16-byte stores need an aligned destination and a stride that keeps every expert aligned; the kernel runs on the
     // current device, so the destination has to be that device's own memory (cudaMemcpy takes any device's)
     int dev;
+    unsigned long long ctx;
     cudaPointerAttributes at;
-    if (!plane || (uintptr_t)dev_dst % 16 || plane % 16 || (dev = current_device()) < 0) return UPLOAD_NOT_TAKEN;
+    if (!plane || (uintptr_t)dev_dst % 16 || plane % 16 || (dev = current_device()) < 0 || !(ctx = context_id())) return UPLOAD_NOT_TAKEN;
     if (cudaPointerGetAttributes(&at, dev_dst) != cudaSuccess || at.type != cudaMemoryTypeDevice || at.device != dev) {
         (void)cudaGetLastError();
         return UPLOAD_NOT_TAKEN;
@@ -112,11 +174,14 @@ int upload_repacked(const void *host_blocks, uint64_t plane, uint64_t e0, uint64
     const int threads = (int)min(min((uint64_t)UP_MAX_THREADS, (uint64_t)(hw > 1 ? hw : 1)), (chunks + 1) / 2);
     const Staging staging = staging_take((chunks > 1 ? (uint64_t)threads * 2 : 1) * UP_SLOT_BYTES);
     if (!staging.p) return UPLOAD_NOT_TAKEN;
+    Lanes lanes = lanes_take(dev, ctx);
     std::atomic<uint64_t> next{0};
     std::atomic<int> err{0};
     auto work = [&](int w) {
         cudaError_t e = cudaSetDevice(dev);
         cudaEvent_t ev[2] = {nullptr, nullptr};
+        cudaStream_t &st = lanes.st[w];
+        if (e == cudaSuccess && !st) e = cudaStreamCreate(&st);      // (a blocking stream: it waits for the first byte's copy)
         for (int s = 0; s < 2 && e == cudaSuccess; s++) e = cudaEventCreateWithFlags(&ev[s], cudaEventDisableTiming);
         for (int s = 0, used = 0; e == cudaSuccess && !err.load(std::memory_order_relaxed); s ^= 1, used++) {
             const uint64_t c = next.fetch_add(1);
@@ -126,9 +191,12 @@ int upload_repacked(const void *host_blocks, uint64_t plane, uint64_t e0, uint64
             const int nb = (int)min((uint64_t)UP_SLOT_BLOCKS, n - b0);
             uint8_t *slot = staging.p + (uint64_t)(2 * w + s) * UP_SLOT_BYTES;
             memcpy(slot, src + b0 * 17, (size_t)nb * 17);
-            launch_k(k_repack, dim3((nb + RP_BLOCKS - 1) / RP_BLOCKS), dim3(RP_BLOCKS), 0, cudaStreamLegacy, (const uint4 *)slot, b0, nb, plane,
-                     (uint8_t *)dev_dst);
-            if ((e = cudaGetLastError()) == cudaSuccess) e = cudaEventRecord(ev[s], cudaStreamLegacy);
+            k_repack<<<(nb + RP_BLOCKS - 1) / RP_BLOCKS, RP_BLOCKS, 0, st>>>((const uint4 *)slot, b0, nb, plane, (uint8_t *)dev_dst);
+            if ((e = cudaGetLastError()) == cudaSuccess) e = cudaEventRecord(ev[s], st);
+        }
+        if (st) {                                       // (also before the staging is used again)
+            const cudaError_t es = cudaStreamSynchronize(st);
+            if (e == cudaSuccess) e = es;
         }
         if (e != cudaSuccess) err = (int)e;
         for (int s = 0; s < 2; s++) if (ev[s]) cudaEventDestroy(ev[s]);
@@ -140,9 +208,9 @@ int upload_repacked(const void *host_blocks, uint64_t plane, uint64_t e0, uint64
     } catch (const std::system_error &) {}              // fewer threads: the others take the chunks
     work(0);
     for (int w = 1; w <= started; w++) pool[w].join();
-    cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);   // (also before the staging is used again)
-    if (e == cudaSuccess) e = (cudaError_t)err.load();
-    const cudaError_t ep = staging_put(staging);
+    cudaError_t e = (cudaError_t)err.load();
+    const cudaError_t el = lanes_put(dev, lanes, true), ep = staging_put(staging);
+    if (e == cudaSuccess) e = el;
     if (e == cudaSuccess) e = ep;
     if (e != cudaSuccess) { last_cuda_error() = (int)e; return Q36_MOE_ECUDA; }
     return Q36_MOE_OK;
