@@ -58,7 +58,7 @@ static LayerWs carve(void *base, int T, int E, int k, int D, int FF) {
     w.soffs = (int *)take(8);
     w.elist = (int *)take(n * 4);
     w.pos = (int *)take(n * 4);
-    w.disp = take(route_dispatch_ws_bytes(T, k <= 8 ? k : 8, E));
+    w.disp = take(route_dispatch_ws_bytes(T, k, E));
     w.Xq = (uint8_t *)take(R * D);
     w.Xs = (uint8_t *)take(R * (D / Q36_QK));
     w.Hq = (uint8_t *)take(R * FF);

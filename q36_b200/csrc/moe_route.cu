@@ -938,6 +938,7 @@ uint64_t dispatch_ws_bytes(int n_entries, int n_expert) {
     return n_chunk * n_expert * sizeof(int) + (uint64_t)n_entries * sizeof(unsigned short) + 256;
 }
 uint64_t route_dispatch_ws_bytes(int T, int k, int n_expert) {
+    k = min(k, 8);   // (the layers refuse a larger k; the size queries answer for any, and a chunk holds no token of 513 entries)
     const uint64_t n_chunk = ((uint64_t)T * k + route_chunk(k) - 1) / route_chunk(k);
     return n_chunk * n_expert * sizeof(int) + (uint64_t)T * k * sizeof(unsigned short) + 256;
 }

@@ -41,6 +41,21 @@ def test_stride_and_workspace_sizes(moe):
     assert moe.lib.q36_moe_workspace_bytes(0, 256, 8, 2048, 512) == 0
 
 
+def test_size_queries_answer_for_any_k(moe):
+    """The layers refuse k > 8, the size queries do not judge it: a number comes back (in a child process: a fault would end this one)."""
+    import subprocess
+    import sys
+    code = ("from q36_b200 import moe\nL = moe.lib\n"
+            "for k in (1, 8, 9, 512, 513, 100000):\n"
+            "    assert L.q36_moe_workspace_bytes(4, 256, k, 2048, 512) > 0\n"
+            "    assert L.q36_moe_ep_workspace_bytes(4, 0, 2, 256, k, 2048, 512) > 0\n"
+            "for f in (L.q36_moe_workspace_bytes, L.q36_moe_block_workspace_bytes):\n"
+            "    assert f(4, 256, 0, 2048, 512) == 0 and f(4, 256, -1, 2048, 512) == 0\n"
+            "assert L.q36_moe_ep_workspace_bytes(4, 0, 2, 256, 0, 2048, 512) == 0\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT)
+    assert r.returncode == 0, (r.returncode, r.stderr[-500:])
+
+
 def test_host_repack_matches_oracle(moe, oracle):
     from q36_b200 import synth
     rng = np.random.default_rng(0)
