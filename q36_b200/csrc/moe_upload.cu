@@ -11,11 +11,10 @@
 
 #include <atomic>
 #include <mutex>
-#include <system_error>
-#include <thread>
 #include <utility>
 
 #include "common.cuh"
+#include "host_threads.h"
 #include "kernels.cuh"
 
 namespace q36 {
@@ -201,13 +200,7 @@ int upload_repacked(const void *host_blocks, uint64_t plane, uint64_t e0, uint64
         if (e != cudaSuccess) err = (int)e;
         for (int s = 0; s < 2; s++) if (ev[s]) cudaEventDestroy(ev[s]);
     };
-    std::thread pool[UP_MAX_THREADS];
-    int started = 0;
-    try {
-        for (int w = 1; w < threads; w++, started++) pool[w] = std::thread(work, w);
-    } catch (const std::system_error &) {}              // fewer threads: the others take the chunks
-    work(0);
-    for (int w = 1; w <= started; w++) pool[w].join();
+    run_on_threads<UP_MAX_THREADS>(threads, work);
     cudaError_t e = (cudaError_t)err.load();
     const cudaError_t el = lanes_put(dev, lanes, true), ep = staging_put(staging);
     if (e == cudaSuccess) e = el;
