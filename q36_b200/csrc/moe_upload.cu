@@ -98,14 +98,25 @@ void *driver_fn(const char *name) {
     cudaDriverEntryPointQueryResult q;
     return cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? p : nullptr;
 }
-// id of the calling thread's context (no two contexts of a process have the same one), 0 if it cannot be had
-unsigned long long context_id() {
+// The calling thread's context and its id (no two contexts of a process have the same one); id 0 if it cannot be had.  A program
+// may work in a context of its own instead of the runtime's: its memory is not there for a kernel launched in another one.
+struct Context { CUcontext c; unsigned long long id; };
+Context current_context() {
     static const auto get = (CUresult (*)(CUcontext *))driver_fn("cuCtxGetCurrent");
     static const auto get_id = (CUresult (*)(CUcontext, unsigned long long *))driver_fn("cuCtxGetId");
-    CUcontext c = nullptr;
-    unsigned long long id = 0;
-    if (!get || !get_id || get(&c) != CUDA_SUCCESS || !c || get_id(c, &id) != CUDA_SUCCESS) return 0;
-    return id;
+    Context x = {nullptr, 0};
+    if (!get || !get_id || get(&x.c) != CUDA_SUCCESS || !x.c || get_id(x.c, &x.id) != CUDA_SUCCESS) x.id = 0;
+    return x;
+}
+cudaError_t enter_context(CUcontext c) {
+    static const auto set = (CUresult (*)(CUcontext))driver_fn("cuCtxSetCurrent");
+    return set && set(c) == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidDevice;
+}
+// Is it another context's memory?  (Memory of a pool belongs to none: the context is null then, or the query is refused.)
+bool elsewhere(const void *p, CUcontext c) {
+    static const auto get = (CUresult (*)(void *, CUpointer_attribute, CUdeviceptr))driver_fn("cuPointerGetAttribute");
+    CUcontext owner = nullptr;
+    return get && get(&owner, CU_POINTER_ATTRIBUTE_CONTEXT, (CUdeviceptr)(uintptr_t)p) == CUDA_SUCCESS && owner && owner != c;
 }
 Lanes lanes_take(int dev, unsigned long long ctx) {
     Lanes l = {};
@@ -139,7 +150,7 @@ int upload_release() {
             any = g_lanes[dev].ctx != 0;
         }
         if (!any || (dev != cur && cudaSetDevice(dev) != cudaSuccess)) continue;
-        const cudaError_t e = lanes_put(dev, lanes_take(dev, context_id()), false);
+        const cudaError_t e = lanes_put(dev, lanes_take(dev, current_context().id), false);
         if (el == cudaSuccess) el = e;
         if (dev != cur && cur >= 0) (void)cudaSetDevice(cur);
     }
@@ -157,13 +168,14 @@ int upload_repacked(const void *host_blocks, uint64_t plane, uint64_t e0, uint64
     // 16-byte stores need an aligned destination and a stride that keeps every expert aligned; the kernel runs on the
     // current device, so the destination has to be that device's own memory (cudaMemcpy takes any device's)
     int dev;
-    unsigned long long ctx;
     cudaPointerAttributes at;
-    if (!plane || (uintptr_t)dev_dst % 16 || plane % 16 || (dev = current_device()) < 0 || !(ctx = context_id())) return UPLOAD_NOT_TAKEN;
+    if (!plane || (uintptr_t)dev_dst % 16 || plane % 16 || (dev = current_device()) < 0) return UPLOAD_NOT_TAKEN;
     if (cudaPointerGetAttributes(&at, dev_dst) != cudaSuccess || at.type != cudaMemoryTypeDevice || at.device != dev) {
         (void)cudaGetLastError();
         return UPLOAD_NOT_TAKEN;
     }
+    const Context ctx = current_context();      // (the call above has made one if there was none)
+    if (!ctx.id || elsewhere(dev_dst, ctx.c)) return UPLOAD_NOT_TAKEN;
     const uint8_t *src = (const uint8_t *)host_blocks + e0 * plane * 17;
     // The first byte goes by a plain copy: it waits for the work before it and is refused (a stream capture under way, say)
     // just like the one copy of the whole tensor that the host route makes.
@@ -173,11 +185,11 @@ int upload_repacked(const void *host_blocks, uint64_t plane, uint64_t e0, uint64
     const int threads = (int)min(min((uint64_t)UP_MAX_THREADS, (uint64_t)(hw > 1 ? hw : 1)), (chunks + 1) / 2);
     const Staging staging = staging_take((chunks > 1 ? (uint64_t)threads * 2 : 1) * UP_SLOT_BYTES);
     if (!staging.p) return UPLOAD_NOT_TAKEN;
-    Lanes lanes = lanes_take(dev, ctx);
+    Lanes lanes = lanes_take(dev, ctx.id);
     std::atomic<uint64_t> next{0};
     std::atomic<int> err{0};
     auto work = [&](int w) {
-        cudaError_t e = cudaSetDevice(dev);
+        cudaError_t e = w ? enter_context(ctx.c) : cudaSuccess;
         cudaEvent_t ev[2] = {nullptr, nullptr};
         cudaStream_t &st = lanes.st[w];
         if (e == cudaSuccess && !st) e = cudaStreamCreate(&st);      // (a blocking stream: it waits for the first byte's copy)

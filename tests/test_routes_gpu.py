@@ -55,6 +55,48 @@ def test_uploads_from_several_threads_do_not_disturb_each_other(moe):
         np.testing.assert_array_equal(g.cpu().numpy(), want)
 
 
+_OWN_CONTEXT = """
+import ctypes as C, sys
+import numpy as np
+from q36_b200 import moe
+cu = C.CDLL("libcuda.so.1")
+def ok(rc): assert rc == 0, rc
+ctx, cur, dst = C.c_void_p(), C.c_void_p(), C.c_uint64()
+ok(cu.cuInit(0))
+ok(cu.cuCtxCreate_v2(C.byref(ctx), 0, 0))
+M, K, n = 512, 2048, 8                                  # eight staging slots: several threads
+blocks = np.random.default_rng(0).integers(0, 256, size=(n, M, K // 32, 17), dtype=np.uint8)
+want, got = np.empty(n * moe.expert_stride(M, K), np.uint8), np.empty(n * moe.expert_stride(M, K), np.uint8)
+moe.check(moe.lib.q36_moe_repack_mxfp4(blocks.ctypes.data, K, M, 0, n, want.ctypes.data), "repack")
+ok(cu.cuMemAlloc_v2(C.byref(dst), C.c_size_t(want.size)))
+for i in range(2):
+    moe.check(moe.lib.q36_moe_upload_mxfp4(blocks.ctypes.data, K, M, 0, n, dst.value), "upload")
+    ok(cu.cuCtxGetCurrent(C.byref(cur)))
+    assert cur.value == ctx.value                        # the caller's thread stays in its context
+    ok(cu.cuMemcpyDtoH_v2(C.c_void_p(got.ctypes.data), dst, C.c_size_t(got.size)))
+    assert (got == want).all()
+    moe.check(moe.lib.q36_moe_upload_release(), "release")
+ok(cu.cuMemsetD8_v2(dst, 0, C.c_size_t(got.size)))
+prim = C.c_void_p()
+ok(cu.cuDevicePrimaryCtxRetain(C.byref(prim), 0))
+ok(cu.cuCtxSetCurrent(prim))                             # the memory of one context, uploaded to from another
+moe.check(moe.lib.q36_moe_upload_mxfp4(blocks.ctypes.data, K, M, 0, n, dst.value), "upload")
+ok(cu.cuCtxSetCurrent(ctx))
+ok(cu.cuMemcpyDtoH_v2(C.c_void_p(got.ctypes.data), dst, C.c_size_t(got.size)))
+assert (got == want).all()
+"""
+
+
+def test_upload_in_a_context_of_the_programs_own(moe):
+    """A program may work in a context of its own instead of the runtime's primary one, as with a plain copy."""
+    import os
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-c", _OWN_CONTEXT], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 # gate/up tiles of 32 ff rows while the groups' tiles are at most the SMs (148: 9 groups x 16), 64 up to 18 groups, then 128
 @pytest.mark.parametrize("k,T,se0,se1,shared", [(4, 1, 0, 32, True), (8, 1, 0, 32, True), (8, 1, 0, 32, False), (4, 2, 0, 32, True),
                                                 (2, 3, 0, 32, True), (4, 3, 0, 32, True), (8, 2, 0, 32, True), (4, 4, 0, 32, True),
