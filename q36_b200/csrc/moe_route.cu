@@ -132,12 +132,13 @@ __global__ void k_router_topk(const float *__restrict__ logits, int n_expert, in
 }
 
 // -------------------------------------------------------------- dispatch
-// Stable counting sort of entry ids by expert in two launches.  Entries are cut into chunks of at most DISPATCH_CHUNK;
+// Stable counting sort of entry ids by expert in two or three launches.  Entries are cut into chunks of at most DISPATCH_CHUNK;
 // inside a chunk warp w owns entries [32w, 32w+32).
 //   k_dispatch_count      : per (expert, chunk) counts and each entry's rank among the chunk's earlier entries of the
 //                           same expert; with ROUTE the chunk's tokens are routed by the same block first
 //   k_dispatch_scan_place : one cluster: per expert exclusive scan over its chunks (a warp per expert), scan over the
 //                           experts, then elist / pos of every entry; its first CTA writes the tensor-core work plan
+// A third one places the entries when they are many (k_dispatch_place), or the row quantiser does (k_quant_rows).
 // The order inside a bucket is ascending entry id, one of the orders the
 // engine's atomic k_moe_dispatch (q36_engine.cu:3387-3392) can produce.
 // Bound by latency at every size that matters (12 B per entry).  One block that scanned, and separate router and place
@@ -219,7 +220,7 @@ k_dispatch_scan_place(const int *__restrict__ eid, int n, int per_chunk, int n_e
                       const unsigned short *__restrict__ lrank, int *__restrict__ ecount, int *__restrict__ eoffs,
                       int *__restrict__ elist, int *__restrict__ pos, int *__restrict__ soffs, int s0, int s1, TcPlan *plan, int se0,
                       int se1, int mt_gu, int mt_dn, int plan_tile_rows) {
-    // elist == nullptr: the row quantiser behind this launch places the entries itself (k_quant_rows)
+    // elist == nullptr: a launch behind this one places the entries (k_quant_rows or k_dispatch_place)
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     cluster.barrier_arrive();                 // every CTA has started before anyone writes into its shared memory
@@ -286,6 +287,20 @@ k_dispatch_scan_place(const int *__restrict__ eid, int n, int per_chunk, int n_e
             pos[i] = p;
         }
     }
+}
+
+// elist / pos of many entries, by the whole chip instead of the seven SMs above (see dispatch_launches)
+__global__ void __launch_bounds__(256)
+k_dispatch_place(const int *__restrict__ eid, int n, int per_chunk, const int *__restrict__ cnt_ec, int n_chunk,
+                 const unsigned short *__restrict__ lrank, const int *__restrict__ eoffs, int *__restrict__ elist, int *__restrict__ pos) {
+    Q36_GDS();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const int r = lrank[i], e = eid[i];
+    if (r == 0xffff) { pos[i] = -1; return; }
+    const int p = eoffs[e] + cnt_ec[(size_t)e * n_chunk + i / per_chunk] + r;
+    elist[p] = i;
+    pos[i] = p;
 }
 
 // ------------------------------------------------------------- quantiser
@@ -943,6 +958,11 @@ uint64_t route_dispatch_ws_bytes(int T, int k, int n_expert) {
     return n_chunk * n_expert * sizeof(int) + (uint64_t)T * k * sizeof(unsigned short) + 256;
 }
 
+// Entries up to which the scan's own cluster places them: beyond, a launch over the whole chip costs less than its seven SMs take.
+// us of a dispatch of 256 experts with the placement in the cluster / in a launch of its own (and, before either, with a scan by one
+// block): 512 entries 6.1 / 6.6 (6.0), 4096 entries 7.3 / 7.5 (7.3), 8192 entries 8.7 / 7.6 (7.7), 32,768 entries 12.9 / 9.0 (9.8),
+// 262,144 entries 57.5 / 16.0 (34.2).
+constexpr int PLACE_IN_CLUSTER = 4096;
 // eid == nullptr: the entries are the top-k experts of `logits`, written to idx / wt (per_chunk: whole tokens)
 static int dispatch_launches(const float *logits, int row_stride, int k, float scale, int T, int *idx, float *wt, const int *eid, int n,
                              int n_expert, int se0, int se1, int *ecount, int *eoffs, int *elist, int *pos, void *ws, int *soffs, int s0,
@@ -956,9 +976,13 @@ static int dispatch_launches(const float *logits, int row_stride, int k, float s
         else launch_k(k_dispatch_count<true>, dim3(n_chunk), dim3(1024), 0, st, logits, row_stride, k, scale, T, idx, wt, eid, n, per_chunk,
                       n_expert, se0, se1, cnt_ec, n_chunk, lrank);
     }
-    launch_k_cluster(k_dispatch_scan_place, dim3(1, 1, DISPATCH_CLUSTER), dim3(1024), DISPATCH_CLUSTER, st, eid ? eid : (const int *)idx, n,
-                     per_chunk, n_expert, cnt_ec, n_chunk, (const unsigned short *)lrank, ecount, eoffs, elist, pos, soffs, s0, s1,
-                     (TcPlan *)plan, se0, se1, plan ? FF / TC_M : 0, plan ? D / TC_M : 0, plan_tile_rows);
+    const bool spread = elist && n > PLACE_IN_CLUSTER;
+    if (!eid) eid = idx;
+    launch_k_cluster(k_dispatch_scan_place, dim3(1, 1, DISPATCH_CLUSTER), dim3(1024), DISPATCH_CLUSTER, st, eid, n, per_chunk, n_expert, cnt_ec,
+                     n_chunk, (const unsigned short *)lrank, ecount, eoffs, spread ? nullptr : elist, pos, soffs, s0, s1, (TcPlan *)plan, se0,
+                     se1, plan ? FF / TC_M : 0, plan ? D / TC_M : 0, plan_tile_rows);
+    if (spread) launch_k(k_dispatch_place, dim3((n + 255) / 256), dim3(256), 0, st, eid, n, per_chunk, (const int *)cnt_ec, n_chunk,
+                         (const unsigned short *)lrank, (const int *)eoffs, elist, pos);
     return check_launch();
 }
 int launch_dispatch(const int *eid, int n, int n_expert, int se0, int se1, int *ecount, int *eoffs,
@@ -1028,7 +1052,7 @@ int launch_quant(const void *X, int bf16, uint8_t *Xq, uint8_t *Xs, int T, int K
 }  // namespace q36
 
 // ------------------------------------------------- dispatch without a workspace
-// Scratch of q36_moe_dispatch_noalloc: the per-(chunk, expert) counters and the per-entry ranks of the three
+// Scratch of q36_moe_dispatch_noalloc: the per-(chunk, expert) counters and the per-entry ranks of the
 // dispatch kernels for at most Q36_MOE_NOALLOC_MAX_ENTRIES entries and 512 experts.  It lives in the library
 // image: every GPU that loads the library carries these 96 KiB until the process exits.
 static constexpr int NOALLOC_MAX_ENTRIES = 16384;

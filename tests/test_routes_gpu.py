@@ -131,6 +131,25 @@ def test_gateup_tile_heights_give_the_same_bits(moe):
         assert torch.equal(got, want), f"{n} token(s) per call"
 
 
+# placed by the scan's cluster up to 4096 entries, by a launch of its own beyond; entries of other ranks and without an expert
+@pytest.mark.parametrize("n", [1, 511, 4095, 4096, 4097, 16384, 70001])
+@pytest.mark.parametrize("E,se0,se1", [(256, 0, 256), (64, 16, 48), (512, 100, 512)])
+def test_dispatch_places_every_entry(moe, n, E, se0, se1):
+    import torch
+    rng = np.random.default_rng(n + E)
+    eid = rng.integers(-1, E, size=n, dtype=np.int32)
+    ecount, eoffs, elist, pos = moe.dispatch(torch.from_numpy(eid).cuda(), E, se0, se1)
+    mine = (eid >= se0) & (eid < se1)
+    want_count = np.bincount(eid[mine], minlength=E)
+    want_list = np.flatnonzero(mine)[np.argsort(eid[mine], kind="stable")]
+    want_pos = np.full(n, -1)
+    want_pos[want_list] = np.arange(want_list.size)
+    np.testing.assert_array_equal(ecount.cpu().numpy(), want_count)
+    np.testing.assert_array_equal(eoffs.cpu().numpy(), np.concatenate([[0], np.cumsum(want_count)]))
+    np.testing.assert_array_equal(elist.cpu().numpy()[:want_list.size], want_list)
+    np.testing.assert_array_equal(pos.cpu().numpy(), want_pos)
+
+
 # cluster front end up to 512 tokens (at k = 8), two launches beyond; the decode cluster up to 16
 @pytest.mark.parametrize("E,k", [(256, 8), (128, 6), (64, 1), (32, 8)])
 @pytest.mark.parametrize("T", [16, 17, 63, 64, 65, 511, 512, 513, 1025])
