@@ -60,7 +60,8 @@ int launch_ep_recv_plan(const void *win, uint64_t off_hdr0, uint64_t off_hdr1, u
                         int world, int cap, int row_bytes, int eid_off, unsigned limit, int *status, int n_expert, int se0, int se1,
                         int *ecount, int *eoffs, int *elist, int *pos, int *soffs, int s0, int s1, void *plan, int D, int FF,
                         int plan_tile_rows, int *counts_out, cudaStream_t st);
-// Router + dispatch (+ tensor-core work plan when plan != NULL) in one cluster launch; front_mid_takes: up to 512 tokens
+// Router + dispatch (+ tensor-core work plan when plan != NULL) in one cluster launch; front_mid_takes: 512 tokens at
+// k = 8, 768 at k <= 5
 bool front_mid_takes(int T, int k, int n_expert);
 int launch_front_mid(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1,
                      int *idx, float *wt, int *ecount, int *eoffs, int *elist, int *pos, int *soffs, int s0, int s1,

@@ -535,7 +535,7 @@ __device__ __forceinline__ void sort_entries_block(SortSmem &sm, int e, int n, i
     if (plan) tc_plan_block(sm.s_eoffs + se0, se1 - se0, s1 > s0, s0, s1, plan, mt_gu, mt_dn, sm.scratch, false, plan_tile_rows);
 }
 
-// ------------------------------------------------- front end of up to 512 tokens: one cluster
+// ------------------------------------------------- front end of up to 512 tokens of 8 entries, 768 of fewer: one cluster
 // Router -> stable dispatch -> work plan in ONE launch.  CTA r of the cluster routes the tokens [r tpc, (r + 1) tpc) and
 // counts its entries per expert; the counts (2 B each) go to every CTA's shared memory, so that each of them knows every
 // expert's offset after one cluster barrier and places its own entries.
@@ -626,7 +626,9 @@ k_front_mid(const float *__restrict__ logits, int n_expert, int k, float scale, 
     if (tid < n_expert) {
         ecount[tid] = tot;
         eoffs[tid] = row0;
-        if (plan && tid >= se0 && tid < se1) {   // (groups here hold a few token tiles at most: ranking them by size would buy nothing)
+        if (plan && tid >= se0 && tid < se1) {
+            // (groups in expert order: ranking them by size takes a scan of its own, which did not pay at these sizes, skewed routing
+            // included: see front_mid_takes, the other side of which ranks them)
             const int g = tid - se0;
             plan->row0[g] = row0; plan->cnt[g] = tot; plan->done[g] = 0; plan->order[g] = g;
             plan->base[0][g] = (int)(excl >> 20 & 0xfffff) * mt_gu; plan->base[1][g] = (int)(excl >> 40) * mt_dn;
@@ -712,8 +714,13 @@ int launch_ep_recv_plan(const void *win, uint64_t off_hdr0, uint64_t off_hdr1, u
     return check_launch();
 }
 
+// Tokens bound it as well as entries: its eight SMs route them.  us per layer (256 experts, uniform / skewed routing) through this
+// launch and through the two of launch_route_dispatch: top-4 513 tokens 106.8 / 76.2 and 108.9 / 78.5, 700 tokens 120.5 / 96.4 and
+// 121.5 / 97.8, 800 tokens 134.6 / 108.3 and 135.1 / 107.2, 1024 tokens 151.9 / 90.6 and 149.5 / 90.1; top-1 800 tokens 106.9 / 55.2
+// and 106.7 / 57.0, 1500 tokens 130.6 / 87.9 and 125.7 / 83.8, 4096 tokens 195.5 / 132.4 and 173.1 / 111.4.
+constexpr int FM_MAX_T = 768;
 bool front_mid_takes(int T, int k, int n_expert) {
-    return k >= 1 && k <= 8 && n_expert <= FM_MAX_E && (T + FM_CLUSTER - 1) / FM_CLUSTER * k <= FM_ENTRIES;
+    return T <= FM_MAX_T && k >= 1 && k <= 8 && n_expert <= FM_MAX_E && (T + FM_CLUSTER - 1) / FM_CLUSTER * k <= FM_ENTRIES;
 }
 int launch_front_mid(const float *logits, int n_expert, int k, float scale, int T, int row_stride, int se0, int se1,
                      int *idx, float *wt, int *ecount, int *eoffs, int *elist, int *pos, int *soffs, int s0, int s1,
@@ -1006,7 +1013,7 @@ static void launch_quant_rows(const void *X, int bf16, uint8_t *Xq, uint8_t *Xs,
     if (bf16) launch_k(k_quant_rows<true, PLACE>, dim3(grid), dim3(256), 0, st, X, Xq, Xs, T, K, pos, k, shared_row0, early ? 1 : 0, pl);
     else launch_k(k_quant_rows<false, PLACE>, dim3(grid), dim3(256), 0, st, X, Xq, Xs, T, K, pos, k, shared_row0, early ? 1 : 0, pl);
 }
-// Router, dispatch, plan and the scattered row quantiser of a batch of any size.  Up to 512 tokens one cluster (k_front_mid)
+// Router, dispatch, plan and the scattered row quantiser of a batch of any size.  What front_mid_takes: one cluster (k_front_mid)
 // in front of the quantiser, else the routing count, the scan and the quantiser, which places the entries.
 // Measured (us, router to quantised rows, 256 experts, top-8): 33 tokens 9 against 18 with the kernels this replaces, 96
 // tokens 8 against 22, 300 tokens 15 against 24, 1001 tokens 23 against 31, 4096 tokens 33 against 47.

@@ -150,9 +150,10 @@ def test_dispatch_places_every_entry(moe, n, E, se0, se1):
     np.testing.assert_array_equal(pos.cpu().numpy(), want_pos)
 
 
-# cluster front end up to 512 tokens (at k = 8), two launches beyond; the decode cluster up to 16
-@pytest.mark.parametrize("E,k", [(256, 8), (128, 6), (64, 1), (32, 8)])
-@pytest.mark.parametrize("T", [16, 17, 63, 64, 65, 511, 512, 513, 1025])
+# cluster front end up to 512 tokens at k = 8, 680 at k = 6, 768 at k <= 5, two launches beyond; the decode cluster up to 16
+@pytest.mark.parametrize("E,k,T", [(E, k, T) for E, k in ((256, 8), (128, 6), (64, 1), (32, 8))
+                                   for T in (16, 17, 63, 64, 65, 511, 512, 513, 1025)] +
+                         [(128, 6, 680), (128, 6, 681)] + [(E, k, T) for E, k in ((256, 1), (64, 2), (32, 4), (128, 5)) for T in (768, 769)])
 def test_front_end_of_any_batch(moe, oracle, E, k, T):
     import torch
     rng = np.random.default_rng(T + E)
