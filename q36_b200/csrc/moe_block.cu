@@ -260,6 +260,70 @@ k_router_logits_gemm(const float *__restrict__ W, const float *__restrict__ x, f
     cluster.sync();   // nobody leaves while its partial tile may still be read
 }
 
+// The same for very many tokens: 128 tokens x 64 rows per block, K in chunks of 16 through shared memory (register-prefetched,
+// k-major), 8 x 4 outputs per thread.  With more than two tiles per SM the SMs are full without a split of K, and what counts is
+// warps in flight beside a short inner loop: 79 registers a thread leave room for three blocks, 128 of the kernel above for two.  The rule
+// is in the launcher.
+constexpr int RM_BT = 128;
+__global__ void __launch_bounds__(256)
+k_router_logits_many(const float *__restrict__ W, const float *__restrict__ x, float *__restrict__ logits, int logit_stride,
+                     int n_rows, int T, int D) {
+    Q36_GDS();
+    __shared__ float sx[RG_BK][RM_BT + 4];   // [k][token]
+    __shared__ float sw[RG_BK][RG_BR + 4];   // [k][row]
+    const int t0 = blockIdx.y * RM_BT, r0 = blockIdx.x * RG_BR, tid = threadIdx.x;
+    const int tx = tid & 15, ty = tid >> 4;   // thread tile: tokens ty * 8 .. + 8, rows tx * 4 .. + 4
+    // loaders: x tile 128 x 16 floats = 512 float4 (2 per thread), W tile 64 x 16 = 256 float4 (1 per thread)
+    const int lx_t = tid >> 2, lx_k = (tid & 3) * 4;          // tokens lx_t and lx_t + 64
+    const int lw_r = tid >> 2, lw_k = (tid & 3) * 4;
+    float4 px0, px1, pw;
+    auto fetch = [&](int k0) {
+        const int ta = t0 + lx_t, tb = ta + 64, r = r0 + lw_r;
+        px0 = (ta < T) ? *reinterpret_cast<const float4 *>(x + (size_t)ta * D + k0 + lx_k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        px1 = (tb < T) ? *reinterpret_cast<const float4 *>(x + (size_t)tb * D + k0 + lx_k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        pw = (r < n_rows) ? *reinterpret_cast<const float4 *>(W + (size_t)r * D + k0 + lw_k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto stash = [&]() {
+        sx[lx_k][lx_t] = px0.x; sx[lx_k + 1][lx_t] = px0.y; sx[lx_k + 2][lx_t] = px0.z; sx[lx_k + 3][lx_t] = px0.w;
+        sx[lx_k][lx_t + 64] = px1.x; sx[lx_k + 1][lx_t + 64] = px1.y; sx[lx_k + 2][lx_t + 64] = px1.z; sx[lx_k + 3][lx_t + 64] = px1.w;
+        sw[lw_k][lw_r] = pw.x; sw[lw_k + 1][lw_r] = pw.y; sw[lw_k + 2][lw_r] = pw.z; sw[lw_k + 3][lw_r] = pw.w;
+    };
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+    fetch(0);
+    for (int k0 = 0; k0 < D; k0 += RG_BK) {
+        stash();
+        __syncthreads();
+        if (k0 + RG_BK < D) fetch(k0 + RG_BK);
+#pragma unroll
+        for (int kk = 0; kk < RG_BK; kk++) {
+            const float4 xa = *reinterpret_cast<const float4 *>(&sx[kk][ty * 8]);
+            const float4 xb = *reinterpret_cast<const float4 *>(&sx[kk][ty * 8 + 4]);
+            const float4 wv = *reinterpret_cast<const float4 *>(&sw[kk][tx * 4]);
+            const float xs[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+            const float ws[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(xs[i], ws[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int t = t0 + ty * 8 + i;
+        if (t >= T) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int r = r0 + tx * 4 + j;
+            if (r < n_rows) logits[(size_t)t * logit_stride + r] = acc[i][j];
+        }
+    }
+}
+
 // ------------------------------------------------------------------- after
 // One block per token: the weighted combine in slot order (as k_combine), then the residual add and the next
 // RMSNorm while the row is in registers.  EARLY_META: see k_combine (moe_gemv.cu).
@@ -345,12 +409,19 @@ int launch_pre_norm_router(float *h, const float *a, const float *norm_w, float 
         if (D % RG_BK) return Q36_MOE_EINVAL;
         const int rows = (gate_row == n_rows - 1) ? n_rows - 1 : n_rows;   // the gate row is done already when it is the last one
         if (gate_row >= 0 && gate_row != n_rows - 1) return Q36_MOE_EINVAL;
-        // Tile and split of K: small tiles and eight CTAs per tile until the tiles alone fill the chip; few tiles of a large
-        // batch are still split in four so that the last wave is short (T = 8192: 256 tiles on 148 SMs).
-        const int bt = T <= 128 ? 32 : T <= 1024 ? 64 : 128;
-        const int tiles = ((rows + RG_BR - 1) / RG_BR) * ((T + bt - 1) / bt);
-        const int chunks = D / RG_BK, z = tiles <= sm_count() && chunks >= 8 ? 8 : tiles <= 4 * sm_count() && chunks >= 4 ? 4 : 1;
-        const dim3 grid((rows + RG_BR - 1) / RG_BR, (T + bt - 1) / bt, z);
+        // Tile and split of K: small tiles and eight CTAs per tile until the tiles alone fill the chip; the tiles of a larger batch
+        // are still split in four so that the last wave is short (T = 8192: 256 tiles on 148 SMs).  From 2.2 tiles per SM on the
+        // unsplit kernel with more warps: us with the split one / with that one at 257 rows: 9600 tokens (300 tiles) 330 / 360,
+        // 10,500 (332) 367 / 362, 12,000 402 / 366, 16,384 545 / 494, 20,000 659 / 602, 65,536 2092 / 1674.
+        const int bt = T <= 128 ? 32 : T <= 1024 ? 64 : 128, row_tiles = (rows + RG_BR - 1) / RG_BR;
+        const long tiles = (long)row_tiles * ((T + bt - 1) / bt);
+        if (bt == RM_BT && tiles * 5 > (long)sm_count() * 11) {
+            launch_k(k_router_logits_many, dim3(row_tiles, (T + bt - 1) / bt), dim3(256), 0, st, router_w, (const float *)x, logits, logit_stride,
+                     rows, T, D);
+            return check_launch();
+        }
+        const int chunks = D / RG_BK, z = tiles <= sm_count() && chunks >= 8 ? 8 : chunks >= 4 ? 4 : 1;
+        const dim3 grid(row_tiles, (T + bt - 1) / bt, z);
         const float *xc = x;
         if (bt == 32) launch_k_cluster(k_router_logits_gemm<32, 4, 1>, grid, dim3(64), z, st, router_w, xc, logits, logit_stride, rows, T, D);
         else if (bt == 64) launch_k_cluster(k_router_logits_gemm<64, 4, 1>, grid, dim3(128), z, st, router_w, xc, logits, logit_stride, rows, T, D);

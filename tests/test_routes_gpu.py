@@ -197,9 +197,10 @@ def test_router_rows_without_a_largest_value(moe):
         assert int(idx.min()) >= 0 and int(idx.max()) < E
 
 
-# the logits kernels: rows in registers (1, 2, 4, 8, 16 tokens), then 32-, 64- and 128-token tiles with K split 8, 4 or 1 ways
+# the logits kernels: rows in registers (1, 2, 4, 8, 16 tokens), then 32-, 64- and 128-token tiles with K split 8 or 4 ways, and from
+# 2.2 tiles per SM on (326 tiles of 128 x 64) unsplit
 @pytest.mark.parametrize("T,n_rows", [(1, 33), (2, 257), (3, 65), (5, 257), (9, 129), (16, 257), (17, 257), (33, 33), (128, 257), (129, 129),
-                                      (1000, 257), (1025, 257), (4097, 33), (20000, 257)])
+                                      (1000, 257), (1025, 257), (4097, 33), (10368, 257), (10369, 257), (20000, 257), (41601, 33)])
 def test_router_logits_at_the_changes_of_tile(moe, T, n_rows):
     import torch
     g = torch.Generator(device="cuda")
