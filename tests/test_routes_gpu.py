@@ -17,11 +17,15 @@ def rel_l2(a, b):
     return float((a - b).norm() / b.norm())
 
 
-# one block short of, at and past a 256-block CTA and a 32,768-block staging slot; several slots; a stride or a destination
-# that 16-byte stores cannot take (the host route)
+# the host route: fewer than 16,384 blocks; a stride or a destination that 16-byte stores cannot take.  The device's: from 16,384
+# blocks on; a last CTA of 16, 240 and 256 of its 256 blocks; one block row short of, at and past a 32,768-block staging slot; several
+# slots; experts that end inside a CTA
 @pytest.mark.parametrize("M,K,e0,e1,offset", [(16, 32, 0, 1, 0), (16, 32, 2, 5, 0), (240, 32, 0, 1, 0), (256, 32, 0, 1, 0), (272, 32, 0, 3, 0),
                                               (2047 * 16, 32, 0, 1, 0), (2048 * 16, 32, 0, 1, 0), (2049 * 16, 32, 0, 2, 0),
-                                              (512, 2048, 1, 12, 0), (17, 32, 0, 3, 0), (16, 96, 0, 2, 0), (16, 32, 0, 3, 8)])
+                                              (512, 2048, 1, 12, 0), (17, 32, 0, 3, 0), (16, 96, 0, 2, 0), (16, 32, 0, 3, 8),
+                                              (1023 * 16, 32, 0, 1, 0), (1024 * 16, 32, 0, 1, 0), (1025 * 16, 32, 0, 1, 0),
+                                              (1039 * 16, 32, 0, 1, 0), (1040 * 16, 32, 0, 1, 0), (16, 32, 3, 1027, 0), (48, 96, 2, 177, 0),
+                                              (1025 * 16, 32, 0, 2, 8), (4097, 128, 0, 1, 0)])
 def test_upload_equals_the_host_repack(moe, M, K, e0, e1, offset):
     import torch
     rng = np.random.default_rng(M + K)
