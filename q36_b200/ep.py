@@ -164,6 +164,24 @@ def _layer_args(m, ly, X, logits, out, ws):
             out.data_ptr(), X.shape[0], ws.data_ptr(), ws.numel(), m.stream_ptr())
 
 
+def native_launches(lib, T: int, k: int, world: int, E: int, D: int, FF: int, cap_rows: int = 0, transport: int = TRANSPORT_PEER) -> int:
+    """Kernels that one rank's native layer step launches for a window opened for T tokens and called with T."""
+    n, cap, per = T * k, cap_rows or T * k, E // world
+    S = world * cap
+    one_launch = bool(lib.q36_moe_one_launch_fits(S + T, per, D, FF)) and (world * T <= 16 or S + T <= lib.q36_moe_one_launch_rows())
+    reduced = not one_launch and transport == TRANSPORT_PEER and world <= 8 and T <= cap
+
+    def dispatch(entries):                  # count, scan (+ a launch that places many entries)
+        return 2 + (entries > 4096)
+
+    if not reduced and T <= 16 and n <= 128 and D % 1024 == 0 and D * T <= 32 * 1024:
+        front = 1                           # one cluster routes, sorts, quantises and sends
+    else:
+        front = (1 if T <= 768 and -(-T // 8) * k <= 512 else dispatch(n)) + 2      # + quantise, send
+    plan = 1 if S <= 1024 else 1 + dispatch(S)
+    return front + plan + 1 + (1 if one_launch else 3) + 1       # unpack; expert kernel(s) (+ return); combine
+
+
 class NativeEP:
     """One process per GPU.  The C entry point q36_moe_ep_layer issues the whole step from native code on the
     current stream: the library's kernels store routed rows and result rows straight into the peer ranks'
@@ -175,13 +193,7 @@ class NativeEP:
         from . import moe
         self.moe, self.layers, self.world, self.rank, self.T = moe, layers, world, rank, T
         ly = layers[0]
-        # kernels per layer step: front (cluster at decode sizes, else router + dispatch x3 + quantise), send, the
-        # received slots' plan, unpack, FFN (one launch up to q36_moe_one_launch_rows() rows, else two), return, combine
-        small_front = T <= 16 and T * ly.k <= 128
-        S = world * (cap_rows or T * ly.k)
-        one_launch = S + T <= moe.lib.q36_moe_one_launch_rows()
-        self.launches_per_layer = (1 if small_front else (2 if T * ly.k <= 1024 else 6)) + 1 + (1 if S <= 1024 else 5) + 1 + \
-            (1 if one_launch else 2) + 1 + 1
+        self.launches_per_layer = native_launches(moe.lib, T, ly.k, world, ly.E, ly.D, ly.FF, cap_rows, transport)
         dev = ly.device
         idt = torch.zeros(128, dtype=torch.uint8)
         if rank == 0:

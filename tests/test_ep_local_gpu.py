@@ -184,3 +184,47 @@ def test_a_wait_that_nothing_satisfies_ends_with_a_status(moe, full):
         assert bool(torch.isfinite(ref).all())
     finally:
         loc.close()
+
+
+# one cluster; one-cluster front without and with the received slots' one-block plan; two launches; their place launch; two FFN launches
+@pytest.mark.parametrize("world,T", [(2, 1), (2, 16), (2, 17), (2, 64), (4, 33), (2, 448), (2, 513), (4, 1100)])
+def test_the_stated_launches_are_the_launches(moe, full, world, T):
+    import torch
+    from cuda.bindings import runtime as rt
+    from q36_b200 import ep
+    shards = _shards(moe, full, world)
+    loc = ep.LocalEP(world, [0] * world, T, E, K8, D, FF)
+    try:
+        Xs, Ls = _inputs(world, T, 900)
+        outs = [torch.empty((T, D), device="cuda") for _ in range(world)]
+        loc.layer(shards, Xs, Ls, outs)
+        torch.cuda.synchronize()
+        graph, stream = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+        with torch.cuda.stream(stream), torch.cuda.graph(graph, stream=stream):
+            loc.layer(shards, Xs, Ls, outs)
+        g = rt.cudaGraph_t(graph.raw_cuda_graph())
+        _, _, n = rt.cudaGraphGetNodes(g)
+        _, nodes, _ = rt.cudaGraphGetNodes(g, n)
+        kernels = sum(rt.cudaGraphNodeGetType(x)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for x in nodes)
+        assert kernels == world * ep.native_launches(moe.lib, T, K8, world, E, D, FF)
+    finally:
+        loc.close()
+
+
+@pytest.mark.parametrize("T", [1, 2, 3])
+def test_a_few_tokens_give_the_bits_of_the_single_gpu_layer(moe, full, T):
+    """The single-GPU layer cuts its gate/up tiles by the number of groups, the expert-parallel step does not: the sums are the same."""
+    import torch
+    from q36_b200 import ep
+    shards = _shards(moe, full, 2)
+    loc = ep.LocalEP(2, [0, 0], T, E, K8, D, FF)
+    try:
+        Xs, Ls = _inputs(2, T, 77)
+        outs = [torch.empty((T, D), device="cuda") for _ in range(2)]
+        loc.layer(shards, Xs, Ls, outs)
+        torch.cuda.synchronize()
+        for r in range(2):
+            assert loc.status(r) == moe.OK
+            assert torch.equal(outs[r], full.forward(Xs[r], Ls[r]))
+    finally:
+        loc.close()
