@@ -6,8 +6,10 @@
 //   after   moe = combine(...); h += moe; x_next = rmsnorm(h) * w_next
 //           k_moe_combine(_pf) (q36_engine.cu:785-791, 3393-3401) + k_add_rmsnorm (:696-706, :1966)
 //
-// The router logits are f32 dot products at every batch size (the engine's batched path rounds both operands
-// to fp16 for its wmma GEMM; f32 keeps decode and prefill routing identical).
+// The router logits are f32 dot products at every batch size (the engine's batched path rounds both operands to fp16 for its
+// wmma GEMM).  The order of a dot product's additions follows the batch: one up to 16 tokens, K cut in eight or four pieces in
+// the split kernel (and over two groups of warps from 1025 tokens on), one run over K beyond 2.2 tiles per SM.  So the same token
+// may get logits that differ in the last bits in two batches, and another expert where two tie to these.
 #include <cooperative_groups.h>
 
 #include "common.cuh"

@@ -745,8 +745,8 @@ int launch_front_mid(const float *logits, int n_expert, int k, float scale, int 
 //   CTA 0        router -> stable dispatch -> work plan of the fused tensor-core kernel
 //   CTAs 1..7    quantise the token rows (needs no routing result), wait at the cluster barrier for CTA 0's
 //                row positions, then write every block to the k + 1 rows it feeds.
-// Same results as k_front_small + k_quant_e4m3<., true>: the same route_row, the same ascending-entry order
-// inside an expert's bucket, the same quantiser.
+// Same results as k_front_mid + k_quant_rows: the same route_row, the same ascending-entry order inside an expert's
+// bucket, the same quantiser.  The plan is cut in the decode kernel's 16-row token tiles, whatever launch follows.
 constexpr int FD_CLUSTER = 8;
 constexpr int FD_THREADS = 1024;
 constexpr int FD_MAX_ENTRIES = 128;

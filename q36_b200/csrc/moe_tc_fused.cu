@@ -80,7 +80,8 @@ struct FusedCfg {
     static constexpr int MAX_GROUPS = DISPATCH_MAX_GROUPS + 1;   // the plan lists every group, empty ones included
     static constexpr int MAX_TILES = 192;                // per CTA
     static constexpr int TILE_ROWS = 16;                 // token rows per tile: the plan must be cut for this
-    static constexpr int EXTRA_DOWN = 3 / RS;                 // extra down tiles of a CTA that is one gate/up tile short
+    static constexpr int EXTRA_DOWN = 3;                 // extra down tiles of a CTA that is one gate/up tile short (shorter tiles are
+                                                         // chosen where one round holds them all: no CTA is short of another then)
 };
 static_assert(FusedCfg<1>::STAGE_BYTES % 1024 == 0 && FusedCfg<2>::STAGE_BYTES % 1024 == 0 && FusedCfg<4>::STAGE_BYTES % 1024 == 0, "stage alignment");
 
@@ -610,6 +611,7 @@ int launch_ffn_fused_small(const void *Wg, const void *Wu, const void *Wd, const
     // layers of 41 groups 706 / 707 / 829.
     const int groups = min(R_max, n_group + 1);
     const long tiles = (groups + (long)(R_max - groups) / FusedCfg<1>::TILE_ROWS) * (FF / TC_M);   // (an upper bound)
+    // (The expert-parallel step keeps 128 rows: its R_max is the window's capacity, and nothing was measured there.)
     const int rs = ep ? 1 : tiles * 4 <= sm_count() ? 4 : tiles * 2 <= sm_count() ? 2 : 1;
     auto run = rs == 4 ? run_ffn_fused<4> : rs == 2 ? run_ffn_fused<2> : run_ffn_fused<1>;
     return run(Wg, Wu, Wd, Sg, Su, Sd, n_group, R_max, Xq, Xs, Hq, Hs, Y, D, FF, plan, status, ep, st);

@@ -4,8 +4,9 @@
 // The device does the re-arrangement.  The blocks go into pinned staging as they are (host threads, each with two slots of
 // its own) and k_repack reads a slot over PCIe, 16 bytes per thread, and writes codes and scales where they belong: no
 // second host copy, no device staging, and the threads' copies overlap the transfer.  What bounds it is then the PCIe
-// link and the host's copy into pinned memory.  A layer of 64 + 1 experts (109 MB, six uploads): 4.7 ms; 47.6 when one
-// host thread took the blocks apart and a pageable copy followed; 45 when every upload pinned its own staging.
+// link and the host's copy into pinned memory.  A layer of 64 + 1 experts (109 MB, six uploads) takes
+// 3.7 to 4.3 ms; 47.6 when one host thread took the blocks apart and a pageable copy followed; 45 when every upload pinned its own
+// staging, as the first one of a process does (3 to 21 ms, once).
 #include <cuda.h>
 #include <string.h>
 
