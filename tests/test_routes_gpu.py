@@ -201,6 +201,52 @@ def test_router_rows_without_a_largest_value(moe):
         assert int(idx.min()) >= 0 and int(idx.max()) < E
 
 
+def _choices(row, k):
+    """The selection rule in plain words: largest first, the lower id among equals, what is NaN or at most -1e30 never; expert 0 fills
+    the slots that stay empty."""
+    ids = [e for e in range(len(row)) if row[e] > -1e30]
+    ids.sort(key=lambda e: (-float(row[e]), e))
+    return (ids + [0] * k)[:k]
+
+
+@pytest.mark.parametrize("E,k", [(32, 8), (64, 4), (128, 1), (256, 8), (256, 3)])
+@pytest.mark.parametrize("T", [12, 40, 600])                 # the decode cluster, the batch cluster, the two launches
+def test_router_choices_by_definition(moe, E, k, T):
+    import torch
+    rng = np.random.default_rng(E + k)
+    L = rng.standard_normal((T, E + 1), dtype=np.float32)
+    low = np.finfo(np.float32).min
+    L[0, :E] = -np.inf
+    L[1, :E] = low
+    L[2, 3] = np.nan
+    L[3, 5:E] = -np.inf
+    L[4, 7] = np.inf
+    L[5, 2:E] = low
+    L[6, :E] = 0.5                                           # every value ties
+    L[7, :E] = np.where(np.arange(E) % 2, 0.0, -0.0)         # ... and these do
+    L[8, E // 4:] = 3.0                                      # more than a warp's worth tie for the first place
+    L[9, :E] = np.float32(-1e30)
+    L[10, :E] = np.nan
+    L[11, :E] = np.sort(L[11, :E])
+    lt = torch.from_numpy(L).cuda()
+    ly = moe.MoELayer(n_expert=E, k=k).random_planes(1)
+    X = torch.from_numpy(synth.activations(rng, T)).cuda()
+    _, idx, wt = ly.forward(X, lt, want_routing=True)
+    ly.check_device_status()
+    sidx, swt = moe.router_topk(lt, E, k)
+    want = np.array([_choices(L[t, :E], k) for t in range(T)])
+    for i, w in ((idx, wt), (sidx, swt)):
+        np.testing.assert_array_equal(i.cpu().numpy(), want)
+        w = w.cpu().numpy()
+        for t in range(T):
+            v = L[t, :E].astype(np.float64)
+            if not np.isfinite(v[want[t]]).all() or not (v > -1e30).any() or np.isnan(v).any():
+                continue
+            e = np.where(np.arange(k) < (v > -1e30).sum(), np.exp(v[want[t]] - v.max()), 0.0)      # an empty slot weighs nothing
+            # exponentials and two quotients in f32: a few ulps each
+            np.testing.assert_allclose(w[t], e / e.sum(), rtol=3e-6, atol=1e-12)
+
+
 # the logits kernels: rows in registers (1, 2, 4, 8, 16 tokens), then 32-, 64- and 128-token tiles with K split 8 or 4 ways, and from
 # 2.2 tiles per SM on (326 tiles of 128 x 64) unsplit
 @pytest.mark.parametrize("T,n_rows", [(1, 33), (2, 257), (3, 65), (5, 257), (9, 129), (16, 257), (17, 257), (33, 33), (128, 257), (129, 129),
